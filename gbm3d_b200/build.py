@@ -16,7 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 SRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgbm3d.so")
-SOURCES = ["match.cu", "wavelet.cu", "wiener.cu", "aggregate.cu", "gbm3d_api.cu", "noalloc.cu", "global_match.cu",
+SOURCES = ["match.cu", "match_bound.cu", "wavelet.cu", "wiener.cu", "aggregate.cu", "gbm3d_api.cu", "noalloc.cu", "global_match.cu",
            "tc_check.cu", "match_tc.cu", "pilot.cu", "video.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -95,6 +95,11 @@ bool match_supported(int d, int d2);
 // the image is not TMA-addressable (16-byte aligned base, P a multiple of 4).
 bool encode_search_map(CUtensorMap* tm, const float* pad, int R, int Q, int P, int box_rows, int box_cols);
 cudaError_t launch_match(int d, int d2, const MatchArgs& A, cudaStream_t st);
+// Patch 8, search 32, top-K branch (match_bound.cu): tensor-core distances
+// bound the candidates, the exact FP32 SSD ranks them; the exhaustive
+// matcher's sets.
+bool match_bound_supported(int d, int d2, const MatchArgs& A);
+cudaError_t launch_match_bound(const MatchArgs& A, cudaStream_t st);
 cudaError_t launch_make_pad(const float* img, int m, int n, int d2, int spin, float* pad, int P,
                             cudaStream_t st);
 cudaError_t launch_gather_volume(const float* pad, int P, int M, int N, int s, int d, int d2, int K, const uint32_t* S,
