@@ -258,13 +258,265 @@ static cudaError_t launch_px_cap(const AggArgs& A, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// List capacity from the expected entries of a tile: (candidate references
-// across the tile's reach) x K, about a quarter of which touch the tile.
+// The same owner-ordered sums, a block at a time (patches 8 and 16).  The
+// kernel above steps the lanes of an 8 x 4 pixel tile through every block that
+// touches the tile: 39 % of its lane slots add something, and every warp filters
+// its CTA's list once per tile.  Here one warp owns RR x RC pixels whose (U, W)
+// sums sit in shared memory, and each lane stands for fixed pixels of the
+// *block*: an entry is one load of the block, and a read, two adds per pixel
+// and a write of the sums, with every lane at work.  The warp applies its entries one
+// after another in the reference's loop order, so every pixel receives the
+// same contributions in the same order and the sums are unchanged.
+//   The region has a border of D pixels in front and D - 1 behind, so a block
+// that overlaps it needs no test per pixel; sums of border pixels are never
+// written out (their owners make them).
+//   PT, the region's column pitch, is 8 modulo 16 pixels of eight bytes: the
+// 8 x 4 pixels of a half patch fall on distinct banks at every block offset.
+//   The warp enumerates the candidates (reference i, j, slot k) whose search
+// window reaches its region, in loop order, and needs no barrier.  A block is
+// 256 (1024) contiguous bytes (group-major), two lines where the image-shaped
+// volume has eight, and is prefetched into L2 when it is listed.
+//   Bounds at 1024^2 dense (ncu): shared-memory pipe 61 %, issue 42-50 %, DRAM
+// 33 %; 272 us per launch against 625 us pixel at a time (of which the
+// group-major layout with its prefetch 310: DRAM reads 2.07 -> 0.72 GB).
+// N floats at p (a multiple of 128 bytes) on their way to L2: an entry's block
+// is loaded only when the list is walked.
+template <int N>
+__device__ __forceinline__ void prefetch_l2(const float* p) {
+#pragma unroll
+  for (int t = 0; t < N; t += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + t));
+}
+
+template <int D, bool KAHAN, int RR, int RC>
+struct AggBlk {
+  static constexpr int PT = D == 8 ? ((RR + 2 * D - 1 + 7) / 16) * 16 + 8 : RR + 2 * D - 1;
+  static constexpr int COLS = RC + 2 * D - 1;
+  static constexpr int SV = KAHAN ? 4 : 2;  // floats per pixel: u, w (and their compensations)
+  static constexpr int NB = D == 8 ? 8 : 4; // entries loaded together
+    static constexpr int EB = 4;              // candidates per lane and enumeration round
+  static constexpr int LC = 2 * 32 * EB;    // list capacity
+  static constexpr size_t BYTES = (size_t)(LC + 2 * NB) * sizeof(int4) + (size_t)PT * COLS * SV * sizeof(float);
+  static_assert(PT >= RR + 2 * D - 1, "pitch");
+};
+
+template <int D, int D2, bool WIE, bool KAHAN, int RR, int RC>
+__global__ void __launch_bounds__(32) k_aggregate_blk(AggArgs A) {
+  using G = AggBlk<D, KAHAN, RR, RC>;
+  constexpr int PT = G::PT, SV = G::SV, NB = G::NB, EB = G::EB;
+  constexpr int NP = D * D / 32, CSTEP = 32 / D;  // pixels per lane, block columns between them
+  constexpr int H = D2 / 2;
+  extern __shared__ int4 smv[];
+  const int lane = threadIdx.x;
+  int4* lst = smv;
+  float* acc = reinterpret_cast<float*>(smv + G::LC + 2 * NB);
+  const unsigned FULL = 0xffffffffu, below = (1u << lane) - 1u;
+  for (int e = lane; e < PT * G::COLS * SV / 4; e += 32) reinterpret_cast<float4*>(acc)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+
+  const int tiles_r = (A.m + RR - 1) / RR, tiles_c = (A.n + RC - 1) / RC;
+  const int tcol = (int)(blockIdx.x / tiles_r) + A.ct0;  // the window's column tiles, modulo the count
+  const int R0 = (blockIdx.x % tiles_r) * RR, C0 = (tcol >= tiles_c ? tcol - tiles_c : tcol) * RC;
+  const int K = A.K, s = A.s;
+  const int PR0 = R0 + H, PC0 = C0 + H;
+  const int i_lo = max(0, ceil_div(PR0 - D - D2 + 2, s)), i_hi = min(A.M - 1, floor_div(PR0 + RR - 1, s));
+  const int j_lo = max(0, ceil_div(PC0 - D - D2 + 2, s)), j_hi = min(A.N - 1, floor_div(PC0 + RC - 1, s));
+  const int NI = i_hi - i_lo + 1, NJ = j_hi - j_lo + 1;
+  const int total = (NI > 0 && NJ > 0) ? NI * NJ * K : 0;
+  const unsigned invK = K > 1 ? (unsigned)(0xFFFFFFFFu / (unsigned)K) + 1u : 0u;  // ceil(2^32 / K)
+  const unsigned invNJ = NJ > 1 ? (unsigned)(0xFFFFFFFFu / (unsigned)NJ) + 1u : 0u;
+
+  // this lane's block pixels: (pr, pc + CSTEP q)
+  const int pr = lane % D, pc = lane / D;
+  const float* vsrc = A.blocks + lane;
+  const float* wsrc = WIE ? A.gw + lane : nullptr;
+  float* apx = acc + (pr + PT * pc) * SV;
+  float mask[NP];
+#pragma unroll
+  for (int q = 0; q < NP; ++q) mask[q] = WIE ? 0.f : A.win[lane + 32 * q];
+
+  struct Batch {
+    int off[NB];  // the block's place in acc
+    float wg[NB], val[NB][NP], wv[NB][WIE ? NP : 1];
+  };
+  auto fetch = [&](Batch& B, int e0) {
+#pragma unroll
+    for (int t = 0; t < NB; ++t) {
+      const int4 en = lst[e0 + t];
+      B.off[t] = en.x;
+      if (!WIE) B.wg[t] = __int_as_float(en.z);
+#pragma unroll
+      for (int q = 0; q < NP; ++q) {
+        B.val[t][q] = __ldg(vsrc + (size_t)(unsigned)(en.y + 32 * q));
+        if (WIE) B.wv[t][q] = __ldg(wsrc + (size_t)(unsigned)(en.z + 32 * q));
+      }
+    }
+  };
+  auto add = [](float& a, float& comp, float x) {
+    const float y = x - comp;
+    const float t = a + y;
+    comp = (t - a) - y;
+    a = t;
+  };
+  auto apply = [&](const Batch& B) {
+#pragma unroll
+    for (int t = 0; t < NB; ++t) {
+      float* p = apx + B.off[t];
+      float dv[NP], dw[NP];
+#pragma unroll
+      for (int q = 0; q < NP; ++q) {
+        dv[q] = WIE ? B.val[t][q] : (B.wg[t] * B.val[t][q]) * mask[q];
+        dw[q] = WIE ? B.wv[t][WIE ? q : 0] : B.wg[t] * mask[q];
+      }
+      if constexpr (KAHAN) {
+        float4 v[NP];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) v[q] = *reinterpret_cast<float4*>(p + PT * CSTEP * q * SV);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          add(v[q].x, v[q].z, dv[q]);
+          add(v[q].y, v[q].w, dw[q]);
+          *reinterpret_cast<float4*>(p + PT * CSTEP * q * SV) = v[q];
+        }
+      } else {
+        float2 v[NP];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) v[q] = *reinterpret_cast<float2*>(p + PT * CSTEP * q * SV);
+#pragma unroll
+        for (int q = 0; q < NP; ++q)
+          *reinterpret_cast<float2*>(p + PT * CSTEP * q * SV) = make_float2(v[q].x + dv[q], v[q].y + dw[q]);
+      }
+      __syncwarp();  // the next entry's pixels may be other lanes' of this one
+    }
+  };
+  // the list, in order; padded to whole batches with entries on the border (offset 0: rows and columns -D .. -1)
+  auto walk = [&](int count) {
+    if (lane < 2 * NB) lst[count + lane] = make_int4(0, 0, 0, 0);
+    __syncwarp();
+    Batch B0, B1;
+    fetch(B0, 0);
+    for (int e0 = 0; e0 < count; e0 += 2 * NB) {
+      fetch(B1, e0 + NB);
+      apply(B0);
+      if (e0 + 2 * NB < count) fetch(B0, e0 + 2 * NB);
+      apply(B1);
+    }
+    __syncwarp();
+  };
+
+  // a round's candidates: index q of the loop order -> (i, j, k), its match
+  // index, its group's count and weight; the next round's loads are in flight
+  // while a round is tested
+  struct Cand {
+    int e[EB], nm[EB];
+    float gw[EB];
+  };
+  auto decode = [&](int q, int& i, int& j, int& k) {
+    // q / K and r2 / NJ by multiply-high with ceil(2^32 / divisor): exact for
+    // dividends below 2^32 / divisor (here below NI NJ K < 2^20)
+    const int r2 = K > 1 ? (int)__umulhi((unsigned)q, invK) : q;
+    const int i2 = NJ > 1 ? (int)__umulhi((unsigned)r2, invNJ) : r2;
+    k = q - r2 * K;
+    i = i_lo + i2;
+    j = j_lo + (r2 - i2 * NJ);
+  };
+  auto look = [&](Cand& C, int base) {
+#pragma unroll
+    for (int u = 0; u < EB; ++u) {
+      int i, j, k;
+      decode(min(base + 32 * u + lane, total - 1), i, j, k);
+      const int g = i + A.M * j;
+      C.nm[u] = A.cnt ? __ldg(A.cnt + g) : K;
+      C.e[u] = (int)__ldg(A.S + (size_t)g * K + k) - 1;
+      C.gw[u] = WIE ? 0.f : __ldg(A.gw + g);
+    }
+  };
+  __syncwarp();
+  int cnt = 0;
+  Cand next;
+  if (total > 0) look(next, 0);
+  for (int base = 0; base < total; base += 32 * EB) {
+    const Cand cur = next;
+    if (base + 32 * EB < total) look(next, base + 32 * EB);
+#pragma unroll
+    for (int u = 0; u < EB; ++u) {
+      int i, j, k;
+      decode(min(base + 32 * u + lane, total - 1), i, j, k);
+      const int e = cur.e[u], r0 = i * s + e % D2 - PR0, c0 = j * s + e / D2 - PC0;
+      const bool hit = base + 32 * u + lane < total && k < cur.nm[u] && r0 > -D && r0 < RR && c0 > -D && c0 < RC;
+      const unsigned bal = __ballot_sync(FULL, hit);
+      if (hit) {
+        const int g = i + A.M * j;
+        int4 en;
+        en.x = (r0 + D + PT * (c0 + D)) * SV;
+        en.y = (g * K + k) * (D * D);
+        en.z = WIE ? g * (D * D) : __float_as_int(cur.gw[u]);
+        en.w = 0;
+        lst[cnt + __popc(bal & below)] = en;
+        prefetch_l2<D * D>(A.blocks + (size_t)(unsigned)en.y);
+      }
+      cnt += __popc(bal);
+    }
+    if (cnt > G::LC - 32 * EB) {
+      walk(cnt);
+      cnt = 0;
+    }
+  }
+  if (cnt) walk(cnt);
+  __syncwarp();
+  for (int e = lane; e < RR * RC; e += 32) {
+    const int r = e % RR, c = e / RR, orow = R0 + r, ocol = C0 + c;
+    if (orow < A.m && ocol < A.n) {
+      const float2 v = *reinterpret_cast<const float2*>(acc + (r + D + PT * (c + D)) * SV);
+      A.U[orow + (size_t)A.m * ocol] = v.x;
+      A.W[orow + (size_t)A.m * ocol] = v.y;
+    }
+  }
+}
+
+template <int D, int D2, bool WIE, bool KAHAN, int RR, int RC>
+static cudaError_t launch_blk(const AggArgs& A, cudaStream_t st) {
+  constexpr size_t sm = AggBlk<D, KAHAN, RR, RC>::BYTES;
+  cudaError_t e = cudaFuncSetAttribute(k_aggregate_blk<D, D2, WIE, KAHAN, RR, RC>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  AggArgs B = A;
+  int nt;
+  tile_span(A.cols, A.n, RC, B.ct0, nt);
+  if (nt == 0) return cudaSuccess;
+  k_aggregate_blk<D, D2, WIE, KAHAN, RR, RC><<<((A.m + RR - 1) / RR) * nt, 32, sm, st>>>(B);
+  return cudaGetLastError();
+}
+
+// Patches 8 and 16 with group-major blocks: block at a time, on the largest
+// region that still gives every SM enough warps to cover the latency of its
+// entries' chain: 24 x 24 (13 resident warps per SM by shared memory) from 10
+// regions per SM on, 16 x 16 from 5, else 8 x 8.  Smaller regions touch more
+// entries per pixel (at stride 8: 0.42 per pixel at 24, 0.52 at 16, 0.88 at 8) but
+// fill the GPU.  Measured, all aggregations of a call in us (pixel-at-a-time
+// kernel / 24 / 16 / 8): 4096^2 at strides 8 / 7 2232 / 1177 / 1394 / 2791; 1024^2 dense
+// 2502 / 1190 / 1340 / 2042; 512^2 reference tiling 131 / 146 / 125 / 175; 301 x 203 dense
+// 590 / 730 / 465 / 318; 128 x 96 77 / 106 / 82 / 69.
+// Otherwise (the median filter's image-shaped volume, other patches): pixel at
+// a time, with the list capacity from the expected entries of a tile:
+// (candidate references across the tile's reach) x K, about a quarter of which
+// touch the tile.
 template <int D, int D2, bool WIE, bool KAHAN = false>
 static cudaError_t launch_px(const AggArgs& A, cudaStream_t st) {
-  const long refs = (long)((CR + D + D2 - 2) / A.s + 1) * ((CC + D + D2 - 2) / A.s + 1);
-  if (refs * A.K / 4 <= 1024 - NTC) return launch_px_cap<D, D2, WIE, KAHAN, 1024>(A, st);
-  return launch_px_cap<D, D2, WIE, KAHAN, 2048>(A, st);
+  if constexpr (D == 8 || D == 16) {
+    if (A.group_major) {
+      auto regions = [&](int r) { return (long)((A.m + r - 1) / r) * ((A.n + r - 1) / r); };
+      if (regions(24) >= 10 * 148) return launch_blk<D, D2, WIE, KAHAN, 24, 24>(A, st);
+      if (regions(16) >= 5 * 148) return launch_blk<D, D2, WIE, KAHAN, 16, 16>(A, st);
+      return launch_blk<D, D2, WIE, KAHAN, 8, 8>(A, st);
+    }
+  }
+  if constexpr (WIE && (D == 8 || D == 16)) {
+    return cudaErrorInvalidValue;  // step 2's blocks are always group-major
+  } else {
+    if (!WIE && A.group_major) return cudaErrorInvalidValue;
+    const long refs = (long)((CR + D + D2 - 2) / A.s + 1) * ((CC + D + D2 - 2) / A.s + 1);
+    if (refs * A.K / 4 <= 1024 - NTC) return launch_px_cap<D, D2, WIE, KAHAN, 1024>(A, st);
+    return launch_px_cap<D, D2, WIE, KAHAN, 2048>(A, st);
+  }
 }
 
 cudaError_t launch_aggregate(const AggArgs& A, cudaStream_t st) {

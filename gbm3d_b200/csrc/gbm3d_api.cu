@@ -541,7 +541,8 @@ struct Spin2Cols {
 };
 
 float* run_wavelet_ht(gbm3d_ctx* c, const float* vol, int m, int n, int K, int levels, int cycleSpin,
-                      const double* tau, const WaveletBank& bk, int filtType, const Spin1Cols* w = nullptr) {
+                      const double* tau, const WaveletBank& bk, int filtType, const Spin1Cols* w = nullptr,
+                      int gs = 0) {
   float* vsum = buf<float>(c, "ht.vsum", (size_t)m * n * K);
   if (filtType == 1) {  // medfilt3 instead of the wavelet (denoiseAndAggregateGPU.m:49-52)
     StageTimer tw(c, 2);
@@ -581,6 +582,7 @@ float* run_wavelet_ht(gbm3d_ctx* c, const float* vol, int m, int n, int K, int l
         o.first = s == 0;
         o.last = s == cycleSpin - 1;
         o.cycles = (float)cycleSpin;
+        o.gs = gs;
       } else {
         o.out = rec[lv];
         o.shift = 0;
@@ -602,10 +604,13 @@ void run_ht(gbm3d_ctx* c, const float* vol, const uint32_t* S, const int32_t* cn
             int d2, int K, int levels, int cycleSpin, const double* tau, const WaveletBank& bk, float* U,
             float* W, int filtType, int s, const Spin1Cols* w = nullptr) {
   const int m = M * d, n = N * d;
-  float* vsum = run_wavelet_ht(c, vol, m, n, K, levels, cycleSpin, tau, bk, filtType, w);
+  // patches 8 and 16: the wavelet's last pass writes each group's blocks contiguous
+  const int gs = filtType != 0 ? 0 : d == 8 ? 3 : d == 16 ? 4 : 0;
+  float* vsum = run_wavelet_ht(c, vol, m, n, K, levels, cycleSpin, tau, bk, filtType, w, gs);
   StageTimer tagg(c, 3);
   float* wgt = buf<float>(c, "ht.wgt", (size_t)M * N);
-  launched(c, launch_ht_weights(vsum, m, n, M, N, d, K, cnt, wgt, c->st, w ? w->weights : ColRange()), "ht_weights");
+  launched(c, launch_ht_weights(vsum, m, n, M, N, d, K, cnt, wgt, c->st, w ? w->weights : ColRange(), gs != 0),
+           "ht_weights");
   AggArgs A{};
   A.S = S;
   A.cnt = cnt;
@@ -616,6 +621,7 @@ void run_ht(gbm3d_ctx* c, const float* vol, const uint32_t* S, const int32_t* cn
   A.K = K;
   A.wiener = 0;
   A.blocks = vsum;
+  A.group_major = gs != 0;
   A.gw = wgt;
   std::vector<double> mk(d * d);
   sine_window(d, 0.1, 0.9, mk.data());
@@ -669,6 +675,7 @@ void run_wiener_agg(gbm3d_ctx* c, WienerArgs& A, int d, int d2, float* U, float*
   G.K = K;
   G.wiener = 1;
   G.blocks = A.out;
+  G.group_major = 1;
   G.gw = A.wt;
   G.s = A.s;
   G.kahan = c->form == 1;

@@ -136,11 +136,15 @@ cudaError_t launch_wav_analysis(const float* in, int Ly, int Lx, int Lz, int shi
 // mode 0: out[p] = v; with shift_out, the value for p lands at p - shift_out.
 // Level-1 cycle-spin accumulation: first (store) / middle (add) / last
 // (add, divide by cycle count, clamp at 0).
+// gs = 0: out is the volume, Oy x Ox x Oz.  gs > 0: out is group-major,
+// [x >> gs][y >> gs][z][x & (2^gs - 1)][y & (2^gs - 1)]: each group's blocks of side
+// 2^gs contiguous, the layout that the weights and the aggregation read.
 struct SynthOut {
   float* out;
   int shift;
   int first, last;
   float cycles;
+  int gs;
 };
 // cols: the output columns (values computed for p, before the shift) to produce.
 cudaError_t launch_wav_synthesis(const float* bands, const float* approx, int Oy, int Ox, int Oz,
@@ -148,10 +152,11 @@ cudaError_t launch_wav_synthesis(const float* bands, const float* approx, int Oy
                                  const ColRange& cols = ColRange());
 // medfilt3 of the volume (filtType 'median').
 cudaError_t launch_medfilt3(const float* V, int m, int n, int K, float* out, cudaStream_t st);
-// Aggregation weight 1/(TV(group)+eps) per group of the image-shaped Vavg.
-// jcols: the group columns (of N) to weigh.
+// Aggregation weight 1/(TV(group)+eps) per group of Vavg (image-shaped, or
+// group-major as SynthOut writes it).  jcols: the group columns (of N) to weigh.
 cudaError_t launch_ht_weights(const float* Vavg, int m, int n, int M, int N, int d, int K,
-                              const int32_t* cnt, float* wgt, cudaStream_t st, const ColRange& jcols = ColRange());
+                              const int32_t* cnt, float* wgt, cudaStream_t st, const ColRange& jcols = ColRange(),
+                              bool group_major = false);
 
 // ---- step 2: empirical Wiener (wiener.cu) --------------------------------------
 struct WienerArgs {
@@ -186,7 +191,10 @@ struct AggArgs {
   int s;                // reference stride (block of reference (i, j) lands at (i s + a, j s + b))
   int kahan;            // 1: Kahan-compensated FP32 sums (precision form; d = 8 only)
   int wiener;           // 0: step-1 weights (scalar x mask); 1: step-2 (precomputed)
-  const float* blocks;  // step 1: tile-space Vavg ((M d) x (N d) x K); step 2: weighted values, d x d x K per group
+  // step 1: Vavg, tile-space ((M d) x (N d) x K) or, with group_major, d x d x K
+  // per group; step 2: weighted values, d x d x K per group
+  const float* blocks;
+  int group_major;
   const float* gw;      // step 1: weight per group; step 2: weight table, d x d per group
   float win[1024];      // step 1: mask (d x d)
   int m, n;             // output size (m = (M-1) s + d, n = (N-1) s + d)

@@ -23,6 +23,19 @@
 
 namespace gbm3d {
 
+// Address parts of a synthesis output: rows (y, z) and columns x, for the two
+// layouts of SynthOut.
+__device__ __forceinline__ size_t synth_row(const SynthOut& o, int y, int z, int Oy, int Ox, int Oz) {
+  if (o.gs == 0) return (size_t)y + (size_t)Oy * Ox * z;
+  return ((size_t)((y >> o.gs) * Oz + z) << (2 * o.gs)) + (y & ((1 << o.gs) - 1));
+}
+__device__ __forceinline__ size_t synth_col_step(const SynthOut& o, int Oy, int Oz) {
+  return o.gs == 0 ? (size_t)Oy : (size_t)((Oy >> o.gs) * Oz) << (2 * o.gs);
+}
+__device__ __forceinline__ size_t synth_col(const SynthOut& o, int x, size_t step) {
+  return (size_t)(x >> o.gs) * step + (size_t)((x & ((1 << o.gs) - 1)) << o.gs);
+}
+
 constexpr int TQ = 32;  // analysis output tile (coefficients per axis)
 constexpr int TP = 32;  // synthesis output tile (samples per axis)
 
@@ -163,7 +176,7 @@ __global__ void __launch_bounds__(256) k_wav_synthesis(const float* __restrict__
       }
     }
     const int oy = pmod(py0 + py - o.shift, Oy), ox = pmod(px0 + px - o.shift, Ox), oz = pmod(pz - o.shift, Oz);
-    float* dst = o.out + oy + (size_t)Oy * (ox + (size_t)Ox * oz);
+    float* dst = o.out + synth_row(o, oy, oz, Oy, Ox, Oz) + synth_col(o, ox, synth_col_step(o, Oy, Oz));
     float v = o.first ? acc : *dst + acc;
     if (o.last) {
       v = v / o.cycles;
@@ -325,7 +338,7 @@ __global__ void __launch_bounds__(256) k_wav_synthesis_dense(const float* __rest
       acc = fmaf(which ? bk.z.s[fz].h[1] : bk.z.s[fz].h[0], X[(fz * TP + px) * TP + py], acc);
     const int oy = wrap_once(py0 + py - o.shift, Oy), ox = wrap_once(px0 + px - o.shift, Ox),
               oz = wrap_once(pz - o.shift, Oz);
-    float* dst = o.out + oy + (size_t)Oy * (ox + (size_t)Ox * oz);
+    float* dst = o.out + synth_row(o, oy, oz, Oy, Ox, Oz) + synth_col(o, ox, synth_col_step(o, Oy, Oz));
     float v = o.first ? acc : *dst + acc;
     if (o.last) {
       v = v / o.cycles;
@@ -628,17 +641,19 @@ __global__ void __launch_bounds__(256, 4) k_wav_synthesis_win(const float* __res
   const int gy = py0 + py;
   if (gy < Oy) {
     const int oy = wrap1(gy - o.shift, Oy);
-    float* r0 = o.out + oy + (size_t)Oy * Ox * pmod(2 * qz - o.shift, Oz);
-    float* r1 = o.out + oy + (size_t)Oy * Ox * pmod(2 * qz - 1 - o.shift, Oz);
+    float* r0 = o.out + synth_row(o, oy, pmod(2 * qz - o.shift, Oz), Oy, Ox, Oz);
+    float* r1 = o.out + synth_row(o, oy, pmod(2 * qz - 1 - o.shift, Oz), Oy, Ox, Oz);
     const int gx0 = px0 + 8 * run;
     int ox = wrap1(gx0 - o.shift, Ox);  // output column of gx0, then stepped by one with wrap
+    const size_t cstep = synth_col_step(o, Oy, Oz);
+    const int cmask = (1 << o.gs) - 1;
+    size_t col = synth_col(o, ox, cstep);
 #pragma unroll
     for (int px = 0; px < 8; ++px) {
       if (gx0 + px < Ox) {
         const float x0 = xv[0][px], x1 = xv[1][px];
         const float v0 = fmaf(fb.szh[0], x1, fmaf(fb.szl[0], x0, 0.f));
         const float v1 = fmaf(fb.szh[1], x1, fmaf(fb.szl[1], x0, 0.f));
-        const size_t col = (size_t)Oy * ox;
         float* d0 = r0 + col;
         float* d1 = r1 + col;
         float a0 = o.first ? v0 : *d0 + v0;
@@ -653,6 +668,7 @@ __global__ void __launch_bounds__(256, 4) k_wav_synthesis_win(const float* __res
         *d1 = a1;
       }
       ox = ox + 1 == Ox ? 0 : ox + 1;
+      col = ox & cmask ? col + (1 << o.gs) : (size_t)(ox >> o.gs) * cstep;
     }
   }
 }
@@ -739,7 +755,8 @@ static cudaError_t launch_synthesis_fast(const float* bands, const float* approx
 // difference array is slot-major, so walking the slots in order keeps each
 // lane's elements (e = lane + 32 t of each array) in increasing e: the sums
 // are the same fixed-order reductions as the generic kernel and the oracle.
-template <int D>
+// GM: V is group-major (SynthOut), else image-shaped m x n x K.
+template <int D, bool GM>
 __global__ void __launch_bounds__(128) k_ht_weights_t(const float* __restrict__ V, int m, int n, int M, int N,
                                                       int K, const int32_t* __restrict__ cnt,
                                                       float* __restrict__ wgt, int g0, int gn) {
@@ -750,13 +767,13 @@ __global__ void __launch_bounds__(128) k_ht_weights_t(const float* __restrict__ 
   if (g < 0) return;
   const int i = g % M, j = g / M;
   const int nm = cnt ? cnt[g] : K;
-  const size_t sz = (size_t)m * n;
-  const float* base = V + (size_t)i * D + (size_t)j * D * m;
+  const size_t sz = GM ? (size_t)SL : (size_t)m * n, cs = GM ? (size_t)D : (size_t)m;
+  const float* base = GM ? V + (size_t)g * K * SL : V + (size_t)i * D + (size_t)j * D * m;
   float tx = 0.f, ty = 0.f, tz = 0.f;
   for (int k = 0; k < nm; ++k) {
     float* cur = sl[warp][k & 1];
     const float* prv = sl[warp][(k & 1) ^ 1];
-    for (int t = lane; t < SL; t += 32) cur[t] = __ldg(base + (t % D) + (size_t)(t / D) * m + sz * k);
+    for (int t = lane; t < SL; t += 32) cur[t] = __ldg(base + (t % D) + (size_t)(t / D) * cs + sz * k);
     __syncwarp();
     // x term: element r + D (c + DM k); this lane's first element of slot k
     for (int e = ((lane - k * SX) % 32 + 32) % 32; e < SX; e += 32) {
@@ -937,6 +954,7 @@ cudaError_t launch_wav_synthesis(const float* bands, const float* approx, int Oy
 // other versions do.  In that layout the slot term's element e sits at e and
 // e + 64, and the x term's at e + 24 k (k = e / 40), so most of the per-term
 // index arithmetic goes away.
+template <bool GM>
 __global__ void __launch_bounds__(128) k_ht_weights_8(const float* __restrict__ V, int m, int n, int M, int N,
                                                       int K, const int32_t* __restrict__ cnt,
                                                       float* __restrict__ wgt, int g0, int gn) {
@@ -948,10 +966,11 @@ __global__ void __launch_bounds__(128) k_ht_weights_8(const float* __restrict__ 
   float* sg = shw + warp * K * SL;
   const int i = g % M, j = g / M;
   const int nm = cnt ? cnt[g] : K;
-  const size_t sz = (size_t)m * n;
+  const size_t sz = GM ? (size_t)SL : (size_t)m * n;
   // lane: row r = lane % 8 of columns lane / 8 and lane / 8 + 4 of every slot
-  const float* p0 = V + (size_t)i * D + (size_t)(j * D + (lane >> 3)) * m + (lane & 7);
-  const float* p1 = p0 + (size_t)4 * m;
+  const float* p0 = GM ? V + (size_t)g * K * SL + lane
+                       : V + (size_t)i * D + (size_t)(j * D + (lane >> 3)) * m + (lane & 7);
+  const float* p1 = p0 + (GM ? (size_t)32 : (size_t)4 * m);
   // slots in batches of 4: eight independent loads in flight per lane
   int k = 0;
   for (; k + 4 <= nm; k += 4) {
@@ -998,27 +1017,28 @@ __global__ void __launch_bounds__(128) k_ht_weights_8(const float* __restrict__ 
 }
 
 cudaError_t launch_ht_weights(const float* Vavg, int m, int n, int M, int N, int d, int K,
-                              const int32_t* cnt, float* wgt, cudaStream_t st, const ColRange& jcols) {
+                              const int32_t* cnt, float* wgt, cudaStream_t st, const ColRange& jcols,
+                              bool group_major) {
   int g0, gn;
   group_span(jcols, M, N, g0, gn);
   if (gn < 0) return cudaSuccess;
   const int G = gn > 0 ? gn : M * N;
-  if (d == 16) {
-    k_ht_weights_t<16><<<(G + 3) / 4, 128, 0, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
-    return cudaGetLastError();
-  }
   if (d == 8) {
     const size_t smb = (size_t)4 * K * 64 * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(k_ht_weights_8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
+    auto kern = group_major ? k_ht_weights_8<true> : k_ht_weights_8<false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
     if (e != cudaSuccess) return e;
-    k_ht_weights_8<<<(G + 3) / 4, 128, smb, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
-    return cudaGetLastError();
+    kern<<<(G + 3) / 4, 128, smb, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
+  } else if (d == 16) {
+    auto kern = group_major ? k_ht_weights_t<16, true> : k_ht_weights_t<16, false>;
+    kern<<<(G + 3) / 4, 128, 0, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
+  } else if (group_major) {
+    return cudaErrorInvalidValue;
+  } else if (d == 32) {
+    k_ht_weights_t<32, false><<<(G + 3) / 4, 128, 0, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
+  } else {
+    k_ht_weights<<<(G + 3) / 4, 128, 0, st>>>(Vavg, m, n, M, N, d, K, cnt, wgt, g0, gn);
   }
-  if (d == 32) {
-    k_ht_weights_t<32><<<(G + 3) / 4, 128, 0, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
-    return cudaGetLastError();
-  }
-  k_ht_weights<<<(G + 3) / 4, 128, 0, st>>>(Vavg, m, n, M, N, d, K, cnt, wgt, g0, gn);
   return cudaGetLastError();
 }
 
