@@ -583,6 +583,8 @@ float* run_wavelet_ht(gbm3d_ctx* c, const float* vol, int m, int n, int K, int l
         o.last = s == cycleSpin - 1;
         o.cycles = (float)cycleSpin;
         o.gs = gs;
+        o.pow2 = (cycleSpin & (cycleSpin - 1)) == 0;
+        o.inv = 1.f / (float)cycleSpin;
       } else {
         o.out = rec[lv];
         o.shift = 0;

@@ -145,6 +145,9 @@ struct SynthOut {
   int first, last;
   float cycles;
   int gs;
+  // cycles a power of two: multiplying by inv = 1 / cycles is the same division
+  int pow2;
+  float inv;
 };
 // cols: the output columns (values computed for p, before the shift) to produce.
 cudaError_t launch_wav_synthesis(const float* bands, const float* approx, int Oy, int Ox, int Oz,

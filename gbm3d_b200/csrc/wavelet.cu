@@ -186,168 +186,6 @@ __global__ void __launch_bounds__(256) k_wav_synthesis(const float* __restrict__
   }
 }
 
-// ---------------------------------------------------------------------------
-// Dense banks: every spatial filter has the taps 0..R and the slot filters
-// the taps 0, 1 (sym4 x Haar, getWaveFilters3D('sym','db',4,1), VBM3D's bank:
-// R = 7).  These are the generic kernels' three passes with the tile shapes
-// and tap loops fixed at compile time, single wraps in place of the modulo
-// (the launcher checks the sizes that make one wrap enough), and in the
-// synthesis y-pass the two output parities of a coefficient pair computed by
-// one thread (the generic pass predicates off half the taps in alternate
-// lanes).  Every output is the same serial fmaf chain, over the same taps in
-// the same order, as in the generic kernels.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ int wrap_once(int v, int L) { return v < 0 ? v + L : (v >= L ? v - L : v); }
-
-// T: coefficients per axis of a CTA's output tile (16: a 22 KB staging area,
-// eight CTAs per SM, where the 32 of the generic kernel allows two).
-template <int R, int T>
-__global__ void __launch_bounds__(256) k_wav_analysis_dense(const float* __restrict__ in, int Ly, int Lx, int Lz,
-                                                            int shift, float* __restrict__ out, WaveletBank bk,
-                                                            LevelBands th, int tx0) {
-  constexpr int TQ = T;
-  constexpr int NY = 2 * TQ + R;
-  extern __shared__ float sm[];
-  float* tz = sm;                // [2][NY(x)][NY(y)]
-  float* tx = sm + 2 * NY * NY;  // [4][TQ(qx)][NY(y)]
-  const int Oy = Ly >> 1, Ox = Lx >> 1, Oz = Lz >> 1;
-  const int ntx = (Ox + TQ - 1) / TQ, bx = blockIdx.y + tx0;
-  const int qy0 = blockIdx.x * TQ, qx0 = (bx >= ntx ? bx - ntx : bx) * TQ, qz = blockIdx.z;
-  const int y0 = 2 * qy0 - R - shift, x0 = 2 * qx0 - R - shift;
-  const size_t plane = (size_t)Ly * Lx;
-  // the slot taps k = 0, 1 read slots (2 qz - k - shift) mod Lz
-  const size_t zo0 = plane * (size_t)wrap_once(2 * qz - shift, Lz);
-  const size_t zo1 = plane * (size_t)wrap_once(2 * qz - 1 - shift, Lz);
-  float hz[2][2];
-#pragma unroll
-  for (int f = 0; f < 2; ++f) {
-    hz[f][0] = bk.z.a[f].h[0];
-    hz[f][1] = bk.z.a[f].h[1];
-  }
-  // load + z-pass (slot axis)
-  for (int e = threadIdx.x; e < NY * NY; e += 256) {
-    const int yy = e % NY, xx = e / NY;
-    const int y = wrap_once(y0 + yy, Ly), x = wrap_once(x0 + xx, Lx);
-    const float* col = in + y + (size_t)Ly * x;
-    const float v0 = col[zo0], v1 = col[zo1];
-#pragma unroll
-    for (int fz = 0; fz < 2; ++fz) tz[fz * NY * NY + e] = fmaf(hz[fz][1], v1, fmaf(hz[fz][0], v0, 0.f));
-  }
-  __syncthreads();
-  // x-pass: the four (fx, fz) combinations as an unrolled outer loop, so
-  // each one's taps are compile-time indices into the bank
-#pragma unroll
-  for (int comb = 0; comb < 4; ++comb) {
-    const Taps& t = bk.xy.a[comb & 1];
-    const float* tzc = tz + (comb >> 1) * NY * NY + R * NY;
-    for (int e = threadIdx.x; e < TQ * NY; e += 256) {
-      const int yy = e % NY, qx = e / NY;
-      const float* src = tzc + yy + 2 * qx * NY;
-      float acc = 0.f;
-#pragma unroll
-      for (int u = 0; u <= R; ++u) acc = fmaf(t.h[u], src[-u * NY], acc);
-      tx[(comb * TQ + qx) * NY + yy] = acc;
-    }
-  }
-  __syncthreads();
-  // y-pass + hard threshold + store: a thread's coefficient (qy, qx) in all
-  // eight bands
-  const size_t bsz = (size_t)Oy * Ox * Oz;
-  for (int e = threadIdx.x; e < TQ * TQ; e += 256) {
-    const int qy = e % TQ, qx = e / TQ;
-    if (qy0 + qy >= Oy || qx0 + qx >= Ox) continue;
-    const float* src0 = tx + qx * NY + 2 * qy + R;
-    float* dst = out + (qy0 + qy) + (size_t)Oy * ((qx0 + qx) + (size_t)Ox * qz);
-#pragma unroll
-    for (int code = 0; code < 8; ++code) {
-      const Taps& t = bk.xy.a[code & 1];
-      const float* src = src0 + (code >> 1) * TQ * NY;
-      float acc = 0.f;
-#pragma unroll
-      for (int u = 0; u <= R; ++u) acc = fmaf(t.h[u], src[-u], acc);
-      if (code) acc = acc * (fabsf(acc) > th.tau[code] ? 1.f : 0.f);
-      dst[code * bsz] = acc;
-    }
-  }
-}
-
-template <int R>
-__global__ void __launch_bounds__(256) k_wav_synthesis_dense(const float* __restrict__ bands,
-                                                             const float* __restrict__ approx, int Oy, int Ox,
-                                                             int Oz, SynthOut o, WaveletBank bk, int tx0) {
-  constexpr int NQ = (TP - 1 + R) / 2 + 1;
-  extern __shared__ float sm[];
-  float* B = sm;               // [8][NQ(qx)][NQ(qy)]
-  float* Y = B + 8 * NQ * NQ;  // [4][NQ(qx)][TP(py)]
-  float* X = Y + 4 * NQ * TP;  // [2][TP(px)][TP(py)]
-  const int Iy = Oy >> 1, Ix = Ox >> 1, Iz = Oz >> 1;
-  const int ntx = (Ox + TP - 1) / TP, bx = blockIdx.y + tx0;
-  const int py0 = blockIdx.x * TP, px0 = (bx >= ntx ? bx - ntx : bx) * TP, qz = blockIdx.z;
-  const int qy0 = py0 >> 1, qx0 = px0 >> 1;
-  const size_t bsz = (size_t)Iy * Ix * Iz;
-
-  for (int e = threadIdx.x; e < 8 * NQ * NQ; e += 256) {
-    const int qyl = e % NQ, qxl = (e / NQ) % NQ, code = e / (NQ * NQ);
-    const int qy = wrap_once(qy0 + qyl, Iy), qx = wrap_once(qx0 + qxl, Ix);
-    const float* src = code ? bands + code * bsz : approx;
-    B[e] = src[qy + (size_t)Iy * (qx + (size_t)Ix * qz)];
-  }
-  __syncthreads();
-  // y-pass: outputs py = 2j (even taps) and 2j + 1 (odd taps) of one thread,
-  // each summing fy = 0 then 1, taps in ascending order
-  for (int e = threadIdx.x; e < 4 * NQ * (TP / 2); e += 256) {
-    const int j = e % (TP / 2), qxl = (e / (TP / 2)) % NQ, comb = e / ((TP / 2) * NQ);
-    float ae = 0.f, ao = 0.f;
-#pragma unroll
-    for (int fy = 0; fy < 2; ++fy) {
-      const float* src = B + (fy + 2 * comb) * NQ * NQ + qxl * NQ + j;
-#pragma unroll
-      for (int u = 0; u <= R; ++u) {
-        const float h = fy ? bk.xy.s[1].h[u] : bk.xy.s[0].h[u];
-        if (u & 1) ao = fmaf(h, src[(u + 1) >> 1], ao);  // (2j + 1 + u) / 2
-        else ae = fmaf(h, src[u >> 1], ae);              // (2j + u) / 2
-      }
-    }
-    *reinterpret_cast<float2*>(Y + (comb * NQ + qxl) * TP + 2 * j) = make_float2(ae, ao);
-  }
-  __syncthreads();
-  // x-pass: combine fx for each fz (px is uniform across a warp)
-  for (int e = threadIdx.x; e < 2 * TP * TP; e += 256) {
-    const int py = e % TP, px = (e / TP) % TP, fz = e / (TP * TP);
-    float acc = 0.f;
-#pragma unroll
-    for (int fx = 0; fx < 2; ++fx) {
-      const float* src = Y + (fx + 2 * fz) * NQ * TP + py;
-#pragma unroll
-      for (int u = 0; u <= R; ++u) {
-        if ((px + u) & 1) continue;
-        acc = fmaf(fx ? bk.xy.s[1].h[u] : bk.xy.s[0].h[u], src[((px + u) >> 1) * TP], acc);
-      }
-    }
-    X[(fz * TP + px) * TP + py] = acc;
-  }
-  __syncthreads();
-  // z-pass: output pz = 2qz takes the slot tap 0 of both bands, pz = 2qz - 1 tap 1
-  for (int e = threadIdx.x; e < 2 * TP * TP; e += 256) {
-    const int py = e % TP, px = (e / TP) % TP, which = e / (TP * TP);
-    if (py0 + py >= Oy || px0 + px >= Ox) continue;
-    const int pz = wrap_once(2 * qz - which, Oz);
-    float acc = 0.f;
-#pragma unroll
-    for (int fz = 0; fz < 2; ++fz)
-      acc = fmaf(which ? bk.z.s[fz].h[1] : bk.z.s[fz].h[0], X[(fz * TP + px) * TP + py], acc);
-    const int oy = wrap_once(py0 + py - o.shift, Oy), ox = wrap_once(px0 + px - o.shift, Ox),
-              oz = wrap_once(pz - o.shift, Oz);
-    float* dst = o.out + synth_row(o, oy, oz, Oy, Ox, Oz) + synth_col(o, ox, synth_col_step(o, Oy, Oz));
-    float v = o.first ? acc : *dst + acc;
-    if (o.last) {
-      v = v / o.cycles;
-      v = v > 0.f ? v : 0.f;
-    }
-    *dst = v;
-  }
-}
-
 // getBM3DAggWeights(3,1) (getBM3DAggWeights.m:11-19) and weight = 1/(D+eps)
 // (denoiseAndAggregateGPU.m:75), one warp per group.  Each of the three sums
 // is a fixed-order reduction: lane l adds the elements l, l+32, ... of the
@@ -402,278 +240,347 @@ __global__ void __launch_bounds__(128) k_ht_weights(const float* __restrict__ V,
 }
 
 // ---------------------------------------------------------------------------
-// Fast path for the two banks GBM3D uses: bior1.5 x Haar (the reference's
-// getWaveFilters3Dbior) and 3D Haar.  Both have the shape
-//   analysis  lo: taps 0..LA-1      hi: taps HA0, HA0+1
-//   synthesis lo: taps SL0, SL0+1   hi: taps 0..SH-1
+// The three separable banks of the pipelines, with tap positions known at
+// compile time:
+//   analysis  lo: taps 0 .. LL-1      hi: taps H0 .. H0+HN-1
+//   synthesis lo: taps S0 .. S0+SN-1  hi: taps 0 .. SH-1
 //   slot axis: taps 0, 1 for all four filters
-// (bior: LA=SH=10, HA0=SL0=4; Haar: LA=SH=2, HA0=SL0=0).  With the tap
-// positions known at compile time every loop unrolls, even and odd outputs
-// are produced together (no divergent parity tests), shared memory rows that
-// a stride-2 filter reads are stored de-interleaved, and no division is left
-// in the inner loops.  Each output is the same serial fmaf chain, in the same
-// tap order, as the generic kernels and the oracle.
+// (bior1.5 x Haar LL = SH = 10, H0 = S0 = 4, HN = SN = 2; 3D Haar all 2 from 0;
+// sym4 x Haar, VBM3D's bank, all 8 from 0).
+//
+// One warp marches along the slow axis x over a strip of the fast axis y, for
+// one pair of slots, with the x window in registers; no block barrier.  A
+// tile-per-CTA version spent 60-70 % of the issue slots, two thirds of them on
+// index arithmetic and on passing every intermediate through shared memory;
+// here a value is loaded once, both x inputs of a step come from registers,
+// and only the y pass (neighbouring lanes) goes through the warp's own piece
+// of shared memory.  Each output is the same serial fmaf chain, over the same taps in
+// the same order, as in the generic kernels and the oracle.  Any size of at
+// least the filter length works (indices wrap modulo the size once per strip),
+// so the small coarse levels run here too.
+//   Measured (all launches of a call, analysis / synthesis): 4096^2 tuned 0.80 -> 0.61 /
+// 0.92 -> 0.61 ms (the floor of one read and one write per voxel is 0.38),
+// dense 21.5 -> 15.4 / 28.2 -> 21.5 ms (floor 10.6 / 13), 128 x 96 with the generic
+// coarse levels 559 -> 113 / 398 -> 114 us, VBM3D at 720p (8 frames) 2.45 -> 1.62 /
+// 4.29 -> 1.83 ms.  At 1024^2 dense level 0 moves its bytes at 62 % (analysis)
+// and 50 % (synthesis) of the copy bandwidth; shared-memory pipe and issue are at 55-65 %
+// at 16 warps per SM (register windows).
 // ---------------------------------------------------------------------------
 struct FastBank {
-  float alo[16], ahi[2], slo[2], shi[16];
+  float alo[10], ahi[10], slo[10], shi[10];
   float azl[2], azh[2], szl[2], szh[2];
 };
 
-__device__ __forceinline__ int wrap1(int v, int L) { return v < 0 ? v + L : (v >= L ? v - L : v); }
+constexpr int MW = 4;  // warps per CTA
+constexpr long MARCH_WARPS = 148 * 32;  // warps that a launch should have, where its size allows
 
-constexpr int FQY = 32, FQX = 16;  // fast analysis tile: coefficients along y (fast axis) and x
+constexpr int imax(int a, int b) { return a > b ? a : b; }
 
-// WIN: the column-tile window of the strip form (tx0); without it the grid
-// covers every tile in order.
-template <int LA, int HA0, bool WIN>
-__global__ void __launch_bounds__(256) k_wav_analysis_fast(const float* __restrict__ in, int Ly, int Lx, int Lz,
-                                                           int shift, float* __restrict__ out, FastBank fb,
-                                                           LevelBands th, int tx0) {
-  constexpr int HALO = LA - 1;
-  constexpr int NY = 2 * FQY + HALO;  // staged rows
-  constexpr int NX = 2 * FQX + HALO;  // staged columns
-  constexpr int NYH = (NY + 1) / 2;   // de-interleaved half rows
-  constexpr int NYHP = ((NYH + 15) / 32) * 32 + 16;  // = 16 mod 32: even and odd rows in different banks
-  constexpr int RT = (NY + 31) / 32;  // row chunks per lane
-  extern __shared__ float sm[];
-  float* tz = sm;                     // [2 fz][NX x][NY y]
-  float* tx = sm + 2 * NX * NY;       // [4 comb][FQX qx][2 parity][NYHP]
+// Analysis.  Lane l holds two neighbouring rows of coefficient row q = q0 + l - HL: 2q and
+// 2q + 1 at an even shift, 2q - 1 and 2q at an odd one, whichever pair starts on 8 bytes in
+// memory.  The HL lanes in front are the halo of the y pass, so a warp makes 32 - HL
+// rows.  Step t loads columns 2 qx - 1 and 2 qx of both slots PD steps ahead, applies the
+// slot pass, then the x pass on the last W columns, and hands the four (fx, fz)
+// results to the neighbouring lanes for the y pass, the threshold and the store.
+template <int LL, int H0, int HN, bool EVEN>
+__global__ void __launch_bounds__(32 * MW, 4) k_wav_analysis_march(const float* __restrict__ in, int Ly, int Lx,
+                                                                   int Lz, int shift, float* __restrict__ out,
+                                                                   FastBank fb, LevelBands th, int ty, int x_lo,
+                                                                   int x_len, int seg) {
+  constexpr int W = imax(LL, H0 + HN), HX = W / 2 - 1, HL = EVEN ? W / 2 : W / 2 - 1;
+  constexpr int U = W > 2 ? W / 2 : 4, PD = 3;
+  static_assert(W % 2 == 0 && (2 * U) % W == 0 && PD < U, "the window repeats every U steps");
+  __shared__ float2 sb[MW][2][4][32 + HL];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int Oy = Ly >> 1, Ox = Lx >> 1, Oz = Lz >> 1;
-  const int ntx = (Ox + FQX - 1) / FQX, bx = WIN ? blockIdx.y + tx0 : blockIdx.y;
-  const int qy0 = blockIdx.x * FQY, qx0 = (WIN && bx >= ntx ? bx - ntx : bx) * FQX, qz = blockIdx.z;
-  const int y0 = 2 * qy0 - HALO - shift, x0 = 2 * qx0 - HALO - shift;
-  const size_t zA = (size_t)Ly * Lx * pmod(2 * qz - shift, Lz), zB = (size_t)Ly * Lx * pmod(2 * qz - 1 - shift, Lz);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int sgi = blockIdx.y, qz = blockIdx.z, strip = blockIdx.x * MW + warp;
+  if (strip >= ty) return;
+  const int q = strip * (32 - HL) - HL + lane;
+  const bool live = lane >= HL && q < Oy;
+  const size_t plane = (size_t)Ly * Lx;
+  // lane offsets stay 32 bits and the rest of every address is the same for the
+  // whole CTA (slots, columns, bands), so it lives in uniform registers
+  const unsigned yo = pmod(EVEN ? 2 * q - shift : 2 * q - 1 - shift, Ly);
+  const float* i0 = in + plane * pmod(2 * qz - shift, Lz);      // slot tap 0
+  const float* i1 = in + plane * pmod(2 * qz - 1 - shift, Lz);  // slot tap 1
+  const int xs = x_lo + sgi * seg, n = min(seg, x_len - sgi * seg), T = n + HX;
+  int xc = pmod(2 * (xs - HX) - 1 - shift, Lx);  // next column to load
+  int ox = xs >= Ox ? xs - Ox : xs;
+  float* dst = out + (size_t)Oy * Ox * qz;
+  const size_t bsz = (size_t)Oy * Ox * Oz;
+  float2(*sw)[4][32 + HL] = sb[warp];
 
-  // stage 1: load the input tile of two slots and apply the slot-axis pass
-  // (warps over columns, lanes over rows)
-  int gy[RT];
+  float2 nx[U][4];   // loaded columns: [2 column + slot], the lane's two rows
+  float w[2][2][W];  // slot-pass results [fz][row][column], a ring of W columns
+  auto load = [&](float2 (&v)[4]) {
 #pragma unroll
-  for (int t = 0; t < RT; ++t) gy[t] = wrap1(y0 + lane + 32 * t, Ly);
-#pragma unroll 3
-  for (int xx = w; xx < NX; xx += 8) {
-    const float* col = in + (size_t)Ly * wrap1(x0 + xx, Lx);
+    for (int c = 0; c < 2; ++c) {
+      v[2 * c] = __ldg(reinterpret_cast<const float2*>(i0 + (size_t)Ly * xc + yo));
+      v[2 * c + 1] = __ldg(reinterpret_cast<const float2*>(i1 + (size_t)Ly * xc + yo));
+      xc = xc + 1 == Lx ? 0 : xc + 1;
+    }
+  };
 #pragma unroll
-    for (int t = 0; t < RT; ++t) {
-      const int yy = lane + 32 * t;
-      if (yy < NY) {
-        const float u0 = __ldg(col + gy[t] + zA), u1 = __ldg(col + gy[t] + zB);  // taps k=0, k=1
-        tz[xx * NY + yy] = fmaf(fb.azl[1], u1, fmaf(fb.azl[0], u0, 0.f));
-        tz[NX * NY + xx * NY + yy] = fmaf(fb.azh[1], u1, fmaf(fb.azh[0], u0, 0.f));
+  for (int p = 0; p < PD; ++p)
+    if (p < T) load(nx[p]);
+  for (int t0 = 0; t0 < T; t0 += U) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + u;
+      if (t >= T) break;
+      if (t + PD < T) load(nx[(u + PD) % U]);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const float2 v0 = nx[u][2 * c], v1 = nx[u][2 * c + 1];
+        w[0][0][(2 * u + c) % W] = fmaf(fb.azl[1], v1.x, fmaf(fb.azl[0], v0.x, 0.f));
+        w[0][1][(2 * u + c) % W] = fmaf(fb.azl[1], v1.y, fmaf(fb.azl[0], v0.y, 0.f));
+        w[1][0][(2 * u + c) % W] = fmaf(fb.azh[1], v1.x, fmaf(fb.azh[0], v0.x, 0.f));
+        w[1][1][(2 * u + c) % W] = fmaf(fb.azh[1], v1.y, fmaf(fb.azh[0], v0.y, 0.f));
+      }
+      if (t >= HX) {
+        // x pass: tap k reads column 2 qx - k, the ring's entry 2u + 1 - k
+        float2 own[4];
+#pragma unroll
+        for (int fz = 0; fz < 2; ++fz) {
+          float lo[2], hi[2];
+#pragma unroll
+          for (int y = 0; y < 2; ++y) {
+            lo[y] = hi[y] = 0.f;
+#pragma unroll
+            for (int k = 0; k < LL; ++k) lo[y] = fmaf(fb.alo[k], w[fz][y][(2 * u + 1 - k + W) % W], lo[y]);
+#pragma unroll
+            for (int k = 0; k < HN; ++k) hi[y] = fmaf(fb.ahi[k], w[fz][y][(2 * u + 1 - H0 - k + W) % W], hi[y]);
+          }
+          own[2 * fz] = make_float2(lo[0], lo[1]);
+          own[2 * fz + 1] = make_float2(hi[0], hi[1]);
+        }
+        float2(*sp)[32 + HL] = sw[t & 1];  // the two halves alternate, so one barrier per step does
+#pragma unroll
+        for (int comb = 0; comb < 4; ++comb) sp[comb][lane + HL] = own[comb];
+        __syncwarp();
+        // y pass: tap k reads row 2q - k
+        float* d = dst + (size_t)Oy * ox;
+#pragma unroll
+        for (int comb = 0; comb < 4; ++comb) {
+          const float2* nb = &sp[comb][lane + HL];
+          float v[W + 1];
+          if (EVEN) {
+            v[0] = own[comb].x;
+#pragma unroll
+            for (int p = 1; p < HL; ++p) {
+              const float2 f = nb[-p];
+              v[2 * p - 1] = f.y;
+              v[2 * p] = f.x;
+            }
+            v[2 * HL - 1] = nb[-HL].y;
+          } else {
+            v[0] = own[comb].y;
+            v[1] = own[comb].x;
+#pragma unroll
+            for (int p = 1; p <= HL; ++p) {
+              const float2 f = nb[-p];
+              v[2 * p] = f.y;
+              v[2 * p + 1] = f.x;
+            }
+          }
+          float lo = 0.f, hi = 0.f;
+#pragma unroll
+          for (int k = 0; k < LL; ++k) lo = fmaf(fb.alo[k], v[k], lo);
+#pragma unroll
+          for (int k = 0; k < HN; ++k) hi = fmaf(fb.ahi[k], v[H0 + k], hi);
+          if (comb) lo = lo * (fabsf(lo) > th.tau[2 * comb] ? 1.f : 0.f);
+          hi = hi * (fabsf(hi) > th.tau[2 * comb + 1] ? 1.f : 0.f);
+          if (live) {
+            (d + (size_t)(2 * comb) * bsz)[(unsigned)q] = lo;
+            (d + (size_t)(2 * comb + 1) * bsz)[(unsigned)q] = hi;
+          }
+        }
+        ox = ox + 1 == Ox ? 0 : ox + 1;
       }
     }
-  }
-  __syncthreads();
-  // stage 2: pass along the slow axis, lo and hi together from the same inputs.
-  // Item = (fz, run of RX coefficients qx, row yy), lanes over rows; the run's
-  // inputs (staged columns 2 q0 .. 2 (q0 + RX - 1) + HALO) are read once into
-  // registers.
-  constexpr int RX = 8, NRX = FQX / RX, NV = 2 * RX + LA - 2;
-  for (int it = threadIdx.x; it < 2 * NRX * NY; it += 256) {
-    const int yy = it % NY, r = it / NY, run = r % NRX, fz = r / NRX;
-    const int q0 = run * RX;
-    const float* col = tz + fz * NX * NY + yy + 2 * q0 * NY;
-    float v[NV];
-#pragma unroll
-    for (int j = 0; j < NV; ++j) v[j] = col[j * NY];
-    float* dst = tx + (yy & 1) * NYHP + (yy >> 1);
-#pragma unroll
-    for (int q = 0; q < RX; ++q) {
-      float lo = 0.f, hi = 0.f;  // tap k reads input x = 2 qx - k: staged column 2 q + HALO - k of the run
-#pragma unroll
-      for (int k = 0; k < LA; ++k) lo = fmaf(fb.alo[k], v[2 * q + HALO - k], lo);
-#pragma unroll
-      for (int k = 0; k < 2; ++k) hi = fmaf(fb.ahi[k], v[2 * q + HALO - HA0 - k], hi);
-      dst[((0 + 2 * fz) * FQX + q0 + q) * 2 * NYHP] = lo;
-      dst[((1 + 2 * fz) * FQX + q0 + q) * 2 * NYHP] = hi;
-    }
-  }
-  __syncthreads();
-  // stage 3: pass along the fast axis, threshold, store (lanes along qy)
-  const int qy = lane;
-  const size_t bsz = (size_t)Oy * Ox * Oz;
-  const bool row_ok = qy0 + qy < Oy;
-  for (int j = w; j < 4 * FQX; j += 8) {
-    const int qx = j % FQX, comb = j / FQX;
-    if (!row_ok || qx0 + qx >= Ox) continue;
-    const float* src = tx + (comb * FQX + qx) * 2 * NYHP;
-    float v[LA];
-#pragma unroll
-    for (int k = 0; k < LA; ++k) {
-      const int R = HALO - k;  // row 2qy + HALO - k
-      v[k] = src[(R & 1) * NYHP + qy + (R >> 1)];
-    }
-    float lo = 0.f, hi = 0.f;
-#pragma unroll
-    for (int k = 0; k < LA; ++k) lo = fmaf(fb.alo[k], v[k], lo);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) hi = fmaf(fb.ahi[k], v[HA0 + k], hi);
-    const int code_lo = 2 * comb, code_hi = 2 * comb + 1;
-    if (code_lo) lo = lo * (fabsf(lo) > th.tau[code_lo] ? 1.f : 0.f);
-    hi = hi * (fabsf(hi) > th.tau[code_hi] ? 1.f : 0.f);
-    const size_t o = (qy0 + qy) + (size_t)Oy * ((qx0 + qx) + (size_t)Ox * qz);
-    out[code_lo * bsz + o] = lo;
-    out[code_hi * bsz + o] = hi;
   }
 }
 
-constexpr int FSY = 64, FSX = 32;  // fast synthesis tile: samples along y and x
+// Synthesis.  Lane l makes the rows 2q and 2q + 1 of pair q = q0 + l.  Step t has the
+// eight bands' coefficients of column t (rows q0 .. q0 + 31 + HS) in a ring of NST
+// staged columns (cp.async, NST - 1 columns in flight), applies the y pass for the four (fx, fz)
+// and, once HS columns are ahead, the x pass and the slot pass for the column
+// pair t - HS from the register windows.
+//   RMW adds to the sums of earlier cycle spins; PAIR: an even shift, so the two
+// rows are neighbours at an 8-byte boundary.
+__device__ __noinline__ float2 divide2(float2 v, float c) { return make_float2(v.x / c, v.y / c); }
 
-// Synthesis of one level for the bior / Haar banks.  A CTA makes FSY x FSX
-// outputs of the two slots of one qz: the 8 bands' coefficients it needs are
-// staged in shared memory, then each output is the same serial fmaf chain, in
-// the same tap order, as the generic kernel and the oracle.  Each thread
-// produces a run of outputs from one window of coefficients held in
-// registers, so a staged coefficient is read from shared memory about once
-// per run instead of once per tap:
-//   y-pass: a thread makes 16 consecutive outputs (8 even/odd pairs) of one
-//           (band combination, qx) column from 8 + LO lo and 8 + HI hi values;
-//   x-pass: a thread makes 8 consecutive columns of one output row for both
-//           slot bands, then the slot pass and the write/accumulate, in
-//           registers.
-// Row strides of the staged arrays are odd, so lanes that walk neighbouring
-// rows hit distinct banks.  Four CTAs fit an SM by shared memory (46.7 KB
-// each), so the register budget is that of four: up to 64 per thread.
-template <int SL0, int SH>
-__global__ void __launch_bounds__(256, 4) k_wav_synthesis_win(const float* __restrict__ bands,
-                                                           const float* __restrict__ approx, int Oy, int Ox,
-                                                           int Oz, SynthOut o, FastBank fb, int tx0) {
-  constexpr int REACH = SH - 1 > SL0 + 1 ? SH - 1 : SL0 + 1;
-  constexpr int NQY = (FSY - 1 + REACH) / 2 + 1;  // staged coefficients along y
-  constexpr int NQX = (FSX - 1 + REACH) / 2 + 1;  // and along x
-  constexpr int BQ = NQY | 1;                     // row stride of the staged coefficients
-  constexpr int YS = FSY + 1;                     // row stride of the y-pass outputs
-  constexpr int LW = (SL0 + 2) / 2;               // lo reach beyond a pair index (t + LW at most)
-  constexpr int HW = SH / 2;                      // hi reach
-  static_assert(FSY % 16 == 0 && FSX % 8 == 0 && FSY * (FSX / 8) == 256, "tile shape");
-  extern __shared__ float sm[];
-  float* B = sm;                    // [8 code][NQX qx][BQ]
-  float* Y = sm + 8 * NQX * BQ;     // [4 comb][NQX qx][YS]
+template <int S0, int SN, int SH, bool RMW, bool PAIR>
+__global__ void __launch_bounds__(32 * MW, 4) k_wav_synthesis_march(const float* __restrict__ bands,
+                                                                 const float* __restrict__ approx, int Oy, int Ox,
+                                                                 int Oz, SynthOut o, FastBank fb, int ty, int x_lo,
+                                                                 int x_len, int seg) {
+  constexpr int W = imax(S0 + SN, SH), HS = W / 2, RW = HS + 1, NST = 4, PQ = 40;
+  static_assert(W % 2 == 0 && 32 + HS <= PQ && 8 * HS <= 64, "ring");
+  __shared__ float ring[MW][NST][8][PQ];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int Iy = Oy >> 1, Ix = Ox >> 1, Iz = Oz >> 1;
-  const int ntx = (Ox + FSX - 1) / FSX, bx = blockIdx.y + tx0;
-  const int py0 = blockIdx.x * FSY, px0 = (bx >= ntx ? bx - ntx : bx) * FSX, qz = blockIdx.z;
-  const int qy0 = py0 >> 1, qx0 = px0 >> 1;
+  const int sgi = blockIdx.y, qz = blockIdx.z, strip = blockIdx.x * MW + warp;
+  if (strip >= ty) return;
+  const int q0 = strip * 32, q = q0 + lane;
+  const bool live = q < Iy;
   const size_t bsz = (size_t)Iy * Ix * Iz, zoff = (size_t)Iy * Ix * qz;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  constexpr int QT = (NQY + 31) / 32;
+  const int xs = x_lo + sgi * seg, n = min(seg, x_len - sgi * seg), T = n + HS;
+  float(*rb)[8][PQ] = ring[warp];
 
-  // stage the 8 bands (warps over (code, qx) rows, lanes over qy)
-  int qyv[QT];
+  // staging: lane's own row of the eight bands, and its share of the HS rows past them
+  const float* pa = approx + zoff;
+  const float* pb = bands + zoff;
+  const unsigned yo = q % Iy;
+  const float* ph[2];
+  int hd[2];
 #pragma unroll
-  for (int t = 0; t < QT; ++t) qyv[t] = wrap1(qy0 + lane + 32 * t, Iy);
-  for (int qxl = w; qxl < NQX; qxl += 8) {  // the 8 bands' rows of column qx, one band after another
-    const size_t coff = zoff + (size_t)Iy * wrap1(qx0 + qxl, Ix);
-#pragma unroll
-    for (int code = 0; code < 8; ++code) {
-      const float* src = (code ? bands + code * bsz : approx) + coff;
-      float* dst = B + (code * NQX + qxl) * BQ;
-#pragma unroll
-      for (int t = 0; t < QT; ++t) {
-        const int qyl = lane + 32 * t;
-        if (qyl < NQY) cp_async4(dst + qyl, src + qyv[t]);
-      }
-    }
+  for (int h = 0; h < 2; ++h) {
+    const int e = lane + 32 * h, code = e / HS, off = 32 + e % HS;
+    hd[h] = e < 8 * HS ? code * PQ + off : -1;
+    ph[h] = (code && e < 8 * HS ? bands + code * bsz : approx) + zoff + (q0 + off) % Iy;
   }
-  cp_async_wait_all();
-  __syncthreads();
-  // y-pass: item = (comb, run, qx); outputs py = 16 run .. 16 run + 15 of column qx
-  constexpr int NRUN = FSY / 16;
-  for (int it = threadIdx.x; it < 4 * NRUN * NQX; it += 256) {
-    const int qxl = it % NQX, r = it / NQX, run = r % NRUN, comb = r / NRUN;
-    const float* bl = B + ((2 * comb) * NQX + qxl) * BQ + 8 * run;
-    const float* bh = B + ((2 * comb + 1) * NQX + qxl) * BQ + 8 * run;
-    float lw[8 + LW], hw[8 + HW];
+  int xc = xs >= Ix ? xs - Ix : xs;  // next column to stage
+  auto stage = [&](int slot) {
+    float* s = &rb[slot][0][0];
+    const size_t col = (size_t)Iy * xc;
+    cp_async4(s + lane, pa + col + yo);
 #pragma unroll
-    for (int j = 0; j < 8 + LW; ++j) lw[j] = bl[j];
+    for (int code = 1; code < 8; ++code) cp_async4(s + code * PQ + lane, pb + code * bsz + col + yo);
 #pragma unroll
-    for (int j = 0; j < 8 + HW; ++j) hw[j] = bh[j];
-    float* dst = Y + (comb * NQX + qxl) * YS + 16 * run;
+    for (int h = 0; h < 2; ++h)
+      if (hd[h] >= 0) cp_async4(s + hd[h], ph[h] + col);
+    xc = xc + 1 == Ix ? 0 : xc + 1;
+  };
+
+  // outputs: rows 2q, 2q + 1 (lane offsets) and slots 2 qz, 2 qz - 1, shifted back
+  const unsigned oA = (unsigned)synth_row(o, pmod(2 * q - o.shift, Oy), 0, Oy, Ox, Oz);
+  const unsigned oB = (unsigned)synth_row(o, pmod(2 * q + 1 - o.shift, Oy), 0, Oy, Ox, Oz);
+  float* const dz[2] = {o.out + synth_row(o, 0, pmod(2 * qz - o.shift, Oz), Oy, Ox, Oz),
+                        o.out + synth_row(o, 0, pmod(2 * qz - 1 - o.shift, Oz), Oy, Ox, Oz)};
+  const size_t cstep = synth_col_step(o, Oy, Oz);
+  const int cmask = (1 << o.gs) - 1;
+  int ox = pmod(2 * xs - o.shift, Ox);
+  size_t col = synth_col(o, ox, cstep);
+  auto after = [&](int x, size_t c) {  // the column after x
+    return x + 1 == Ox ? (size_t)0 : (x + 1) & cmask ? c + ((size_t)1 << o.gs) : (size_t)((x + 1) >> o.gs) * cstep;
+  };
+
 #pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      float ev = 0.f, od = 0.f;
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int k = SL0 + u;
-        if (k % 2 == 0) ev = fmaf(fb.slo[u], lw[t + k / 2], ev);
-        else od = fmaf(fb.slo[u], lw[t + (k + 1) / 2], od);
-      }
-#pragma unroll
-      for (int k = 0; k < SH; ++k) {
-        if (k % 2 == 0) ev = fmaf(fb.shi[k], hw[t + k / 2], ev);
-        else od = fmaf(fb.shi[k], hw[t + (k + 1) / 2], od);
-      }
-      dst[2 * t] = ev;
-      dst[2 * t + 1] = od;
-    }
+  for (int p = 0; p < NST - 1; ++p) {
+    if (p < T) stage(p);
+    cp_async_commit();
   }
-  __syncthreads();
-  // x-pass for both slot bands, then the slot pass: thread = (run of 8 columns, row py)
-  const int py = threadIdx.x % FSY, run = threadIdx.x / FSY;
-  float xv[2][8];
+  // y-pass results [fz][row][column], lo and hi in x; moved down every step
+  // (unrolling the six-step ring instead of moving it stalled on instruction fetch)
+  float wl[2][2][RW] = {}, wh[2][2][RW] = {};
+  for (int t = 0; t < T; ++t) {
+    cp_async_wait_group<NST - 2>();
+    __syncwarp();  // column t is staged; every lane has left column t - 1
+    if (t + NST - 1 < T) stage((t + NST - 1) % NST);
+    cp_async_commit();
+    // the sums of the earlier cycle spins, in flight over this step's passes
+    const size_t cols[2] = {col, after(ox, col)};
+    float2 prev[2][2];
+    if (RMW && t >= HS && live) {
 #pragma unroll
-  for (int fz = 0; fz < 2; ++fz) {
-    const float* yl = Y + ((2 * fz) * NQX + 4 * run) * YS + py;      // lo in x
-    const float* yh = Y + ((2 * fz + 1) * NQX + 4 * run) * YS + py;  // hi in x
-    float lw[4 + LW], hw[4 + HW];
+      for (int c = 0; c < 2; ++c)
 #pragma unroll
-    for (int j = 0; j < 4 + LW; ++j) lw[j] = yl[j * YS];
-#pragma unroll
-    for (int j = 0; j < 4 + HW; ++j) hw[j] = yh[j * YS];
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      float ev = 0.f, od = 0.f;
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int k = SL0 + u;
-        if (k % 2 == 0) ev = fmaf(fb.slo[u], lw[t + k / 2], ev);
-        else od = fmaf(fb.slo[u], lw[t + (k + 1) / 2], od);
-      }
-#pragma unroll
-      for (int k = 0; k < SH; ++k) {
-        if (k % 2 == 0) ev = fmaf(fb.shi[k], hw[t + k / 2], ev);
-        else od = fmaf(fb.shi[k], hw[t + (k + 1) / 2], od);
-      }
-      xv[fz][2 * t] = ev;
-      xv[fz][2 * t + 1] = od;
-    }
-  }
-  // slot-axis pass: slot 2qz from tap 0, slot 2qz-1 from tap 1; write or accumulate
-  const int gy = py0 + py;
-  if (gy < Oy) {
-    const int oy = wrap1(gy - o.shift, Oy);
-    float* r0 = o.out + synth_row(o, oy, pmod(2 * qz - o.shift, Oz), Oy, Ox, Oz);
-    float* r1 = o.out + synth_row(o, oy, pmod(2 * qz - 1 - o.shift, Oz), Oy, Ox, Oz);
-    const int gx0 = px0 + 8 * run;
-    int ox = wrap1(gx0 - o.shift, Ox);  // output column of gx0, then stepped by one with wrap
-    const size_t cstep = synth_col_step(o, Oy, Oz);
-    const int cmask = (1 << o.gs) - 1;
-    size_t col = synth_col(o, ox, cstep);
-#pragma unroll
-    for (int px = 0; px < 8; ++px) {
-      if (gx0 + px < Ox) {
-        const float x0 = xv[0][px], x1 = xv[1][px];
-        const float v0 = fmaf(fb.szh[0], x1, fmaf(fb.szl[0], x0, 0.f));
-        const float v1 = fmaf(fb.szh[1], x1, fmaf(fb.szl[1], x0, 0.f));
-        float* d0 = r0 + col;
-        float* d1 = r1 + col;
-        float a0 = o.first ? v0 : *d0 + v0;
-        float a1 = o.first ? v1 : *d1 + v1;
-        if (o.last) {
-          a0 = a0 / o.cycles;
-          a0 = a0 > 0.f ? a0 : 0.f;
-          a1 = a1 / o.cycles;
-          a1 = a1 > 0.f ? a1 : 0.f;
+        for (int z = 0; z < 2; ++z) {
+          const float* p = dz[z] + cols[c];
+          prev[c][z] = PAIR ? *reinterpret_cast<const float2*>(p + oA) : make_float2(p[oA], p[oB]);
         }
-        *d0 = a0;
-        *d1 = a1;
+    }
+    const float* s = &rb[t % NST][0][lane];
+#pragma unroll
+    for (int comb = 0; comb < 4; ++comb) {
+      const float* sl = s + 2 * comb * PQ;
+      const float* sh = sl + PQ;
+      float cl[HS + 1], ch[HS + 1];
+#pragma unroll
+      for (int p = 0; p <= HS; ++p) {  // only the entries that taps use are read
+        if (p >= S0 / 2 && p <= (S0 + SN) / 2) cl[p] = sl[p];
+        if (p <= SH / 2) ch[p] = sh[p];
+      }
+      float ev = 0.f, od = 0.f;
+#pragma unroll
+      for (int k = S0; k < S0 + SN; ++k) {
+        if (k % 2 == 0) ev = fmaf(fb.slo[k - S0], cl[k / 2], ev);
+        else od = fmaf(fb.slo[k - S0], cl[(k + 1) / 2], od);
+      }
+#pragma unroll
+      for (int k = 0; k < SH; ++k) {
+        if (k % 2 == 0) ev = fmaf(fb.shi[k], ch[k / 2], ev);
+        else od = fmaf(fb.shi[k], ch[(k + 1) / 2], od);
+      }
+      if (comb & 1) {
+        wh[comb >> 1][0][HS] = ev;
+        wh[comb >> 1][1][HS] = od;
+      } else {
+        wl[comb >> 1][0][HS] = ev;
+        wl[comb >> 1][1][HS] = od;
+      }
+    }
+    if (t >= HS) {
+      // x pass of the column pair j = t - HS: tap k reads column j + ceil(k / 2)
+      float xv[2][2][2];  // [fz][row][even, odd column]
+#pragma unroll
+      for (int fz = 0; fz < 2; ++fz)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          float ev = 0.f, od = 0.f;
+#pragma unroll
+          for (int k = S0; k < S0 + SN; ++k) {
+            if (k % 2 == 0) ev = fmaf(fb.slo[k - S0], wl[fz][y][k / 2], ev);
+            else od = fmaf(fb.slo[k - S0], wl[fz][y][(k + 1) / 2], od);
+          }
+#pragma unroll
+          for (int k = 0; k < SH; ++k) {
+            if (k % 2 == 0) ev = fmaf(fb.shi[k], wh[fz][y][k / 2], ev);
+            else od = fmaf(fb.shi[k], wh[fz][y][(k + 1) / 2], od);
+          }
+          xv[fz][y][0] = ev;
+          xv[fz][y][1] = od;
+        }
+      // slot pass: slot 2 qz from tap 0, slot 2 qz - 1 from tap 1; write or accumulate
+      if (live) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int z = 0; z < 2; ++z) {
+            float2 v = make_float2(fmaf(fb.szh[z], xv[1][0][c], fmaf(fb.szl[z], xv[0][0][c], 0.f)),
+                                   fmaf(fb.szh[z], xv[1][1][c], fmaf(fb.szl[z], xv[0][1][c], 0.f)));
+            if (RMW) v = make_float2(prev[c][z].x + v.x, prev[c][z].y + v.y);
+            if (o.last) {
+              v = o.pow2 ? make_float2(v.x * o.inv, v.y * o.inv) : divide2(v, o.cycles);
+              v = make_float2(v.x > 0.f ? v.x : 0.f, v.y > 0.f ? v.y : 0.f);
+            }
+            float* p = dz[z] + cols[c];
+            if (PAIR) {
+              *reinterpret_cast<float2*>(p + oA) = v;
+            } else {
+              p[oA] = v.x;
+              p[oB] = v.y;
+            }
+          }
       }
       ox = ox + 1 == Ox ? 0 : ox + 1;
-      col = ox & cmask ? col + (1 << o.gs) : (size_t)(ox >> o.gs) * cstep;
+      col = after(ox, cols[1]);
+      ox = ox + 1 == Ox ? 0 : ox + 1;
     }
+#pragma unroll
+    for (int fz = 0; fz < 2; ++fz)
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int p = 0; p < RW - 1; ++p) {
+          wl[fz][y][p] = wl[fz][y][p + 1];
+          wh[fz][y][p] = wh[fz][y][p + 1];
+        }
   }
 }
 
-// Which fast kernel (if any) a bank maps to: 1 = bior shape, 2 = Haar shape.
+// Which compile-time bank a bank is: 1 bior1.5 x Haar, 2 Haar, 3 sym4 x Haar shape; 0 none.
 static bool taps_are(const Taps& t, int first, int count) {
   if (t.n != count) return false;
   for (int u = 0; u < count; ++u)
@@ -684,69 +591,59 @@ static bool taps_are(const Taps& t, int first, int count) {
 static int fast_kind(const WaveletBank& bk) {
   for (int f = 0; f < 2; ++f)
     if (!taps_are(bk.z.a[f], 0, 2) || !taps_are(bk.z.s[f], 0, 2)) return 0;
-  if (taps_are(bk.xy.a[0], 0, 10) && taps_are(bk.xy.a[1], 4, 2) && taps_are(bk.xy.s[0], 4, 2) &&
-      taps_are(bk.xy.s[1], 0, 10))
-    return 1;
-  if (taps_are(bk.xy.a[0], 0, 2) && taps_are(bk.xy.a[1], 0, 2) && taps_are(bk.xy.s[0], 0, 2) &&
-      taps_are(bk.xy.s[1], 0, 2))
-    return 2;
-  return 0;
+  auto is = [&](int al, int ah, int ahn, int sl, int sln, int sh) {
+    return taps_are(bk.xy.a[0], 0, al) && taps_are(bk.xy.a[1], ah, ahn) && taps_are(bk.xy.s[0], sl, sln) &&
+           taps_are(bk.xy.s[1], 0, sh);
+  };
+  return is(10, 4, 2, 4, 2, 10) ? 1 : is(2, 0, 2, 0, 2, 2) ? 2 : is(8, 0, 8, 0, 8, 8) ? 3 : 0;
 }
 
 static FastBank fast_bank(const WaveletBank& bk) {
   FastBank f{};
-  for (int u = 0; u < bk.xy.a[0].n; ++u) f.alo[u] = bk.xy.a[0].h[u];
-  for (int u = 0; u < 2; ++u) {
-    f.ahi[u] = bk.xy.a[1].h[u];
-    f.slo[u] = bk.xy.s[0].h[u];
-    f.azl[u] = bk.z.a[0].h[u];
-    f.azh[u] = bk.z.a[1].h[u];
-    f.szl[u] = bk.z.s[0].h[u];
-    f.szh[u] = bk.z.s[1].h[u];
-  }
-  for (int u = 0; u < bk.xy.s[1].n; ++u) f.shi[u] = bk.xy.s[1].h[u];
+  auto put = [](float* d, const Taps& t) {
+    for (int u = 0; u < t.n; ++u) d[u] = t.h[u];
+  };
+  put(f.alo, bk.xy.a[0]);
+  put(f.ahi, bk.xy.a[1]);
+  put(f.slo, bk.xy.s[0]);
+  put(f.shi, bk.xy.s[1]);
+  put(f.azl, bk.z.a[0]);
+  put(f.azh, bk.z.a[1]);
+  put(f.szl, bk.z.s[0]);
+  put(f.szh, bk.z.s[1]);
   return f;
 }
 
-template <int LA, int HA0, bool WIN>
-static cudaError_t launch_analysis_fast_t(const float* in, int Ly, int Lx, int Lz, int shift, float* out,
-                                        const FastBank& fb, const LevelBands& th, cudaStream_t st,
-                                        const ColRange& qcols) {
-  constexpr int NY = 2 * FQY + LA - 1, NX = 2 * FQX + LA - 1, NYH = (NY + 1) / 2;
-  constexpr int NYHP = ((NYH + 15) / 32) * 32 + 16;
-  const size_t sm = (size_t)(2 * NX * NY + 4 * FQX * 2 * NYHP) * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(k_wav_analysis_fast<LA, HA0, WIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess) return e;
-  int t0, nt;
-  tile_span(qcols, Lx / 2, FQX, t0, nt);
-  if (nt == 0) return cudaSuccess;
-  dim3 grid((Ly / 2 + FQY - 1) / FQY, nt, Lz / 2);
-  k_wav_analysis_fast<LA, HA0, WIN><<<grid, 256, sm, st>>>(in, Ly, Lx, Lz, shift, out, fb, th, t0);
+// Columns per march: long enough to amortise the halo steps (W / 2 columns in
+// front), short enough to give every SM 32 warps: 4 instead of 8 columns at least took 128 x 96
+// from 148 + 137 to 125 + 113 us; 64 warps per SM changed nothing.
+static int march_segment(int len, long strips) {
+  int seg = 64;
+  while (seg > 4 && strips * ((len + seg - 1) / seg) < MARCH_WARPS) seg >>= 1;
+  return seg;
+}
+
+template <int LL, int H0, int HN>
+static cudaError_t launch_analysis_march(const float* in, int Ly, int Lx, int Lz, int shift, float* out,
+                                         const FastBank& fb, const LevelBands& th, cudaStream_t st, int lo, int len) {
+  const bool even = (shift & 1) == 0;
+  const int nout = 32 - (imax(LL, H0 + HN) / 2 - (even ? 0 : 1));
+  const int ty = (Ly / 2 + nout - 1) / nout, seg = march_segment(len, (long)ty * (Lz / 2));
+  const dim3 grid((ty + MW - 1) / MW, (len + seg - 1) / seg, Lz / 2);
+  auto kern = even ? k_wav_analysis_march<LL, H0, HN, true> : k_wav_analysis_march<LL, H0, HN, false>;
+  kern<<<grid, 32 * MW, 0, st>>>(in, Ly, Lx, Lz, shift, out, fb, th, ty, lo, len, seg);
   return cudaGetLastError();
 }
 
-template <int LA, int HA0>
-static cudaError_t launch_analysis_fast(const float* in, int Ly, int Lx, int Lz, int shift, float* out,
-                                        const FastBank& fb, const LevelBands& th, cudaStream_t st,
-                                        const ColRange& qcols) {
-  return qcols.all(Lx / 2) ? launch_analysis_fast_t<LA, HA0, false>(in, Ly, Lx, Lz, shift, out, fb, th, st, qcols)
-                           : launch_analysis_fast_t<LA, HA0, true>(in, Ly, Lx, Lz, shift, out, fb, th, st, qcols);
-}
-
-template <int SL0, int SH>
-static cudaError_t launch_synthesis_fast(const float* bands, const float* approx, int Oy, int Ox, int Oz,
-                                         const SynthOut& o, const FastBank& fb, cudaStream_t st,
-                                         const ColRange& cols) {
-  constexpr int REACH = SH - 1 > SL0 + 1 ? SH - 1 : SL0 + 1;
-  constexpr int NQY = (FSY - 1 + REACH) / 2 + 1, NQX = (FSX - 1 + REACH) / 2 + 1;
-  const size_t sm = ((size_t)8 * NQX * (NQY | 1) + (size_t)4 * NQX * (FSY + 1)) * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(k_wav_synthesis_win<SL0, SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess) return e;
-  int t0, nt;
-  tile_span(cols, Ox, FSX, t0, nt);
-  if (nt == 0) return cudaSuccess;
-  dim3 grid((Oy + FSY - 1) / FSY, nt, Oz / 2);
-  k_wav_synthesis_win<SL0, SH><<<grid, 256, sm, st>>>(bands, approx, Oy, Ox, Oz, o, fb, t0);
+template <int S0, int SN, int SH>
+static cudaError_t launch_synthesis_march(const float* bands, const float* approx, int Oy, int Ox, int Oz,
+                                          const SynthOut& o, const FastBank& fb, cudaStream_t st, int lo, int len) {
+  const int ty = (Oy / 2 + 31) / 32, seg = march_segment(len, (long)ty * (Oz / 2));
+  const dim3 grid((ty + MW - 1) / MW, (len + seg - 1) / seg, Oz / 2);
+  const bool pair = (o.shift & 1) == 0;
+  auto kern = o.first ? (pair ? k_wav_synthesis_march<S0, SN, SH, false, true> : k_wav_synthesis_march<S0, SN, SH, false, false>)
+                      : (pair ? k_wav_synthesis_march<S0, SN, SH, true, true> : k_wav_synthesis_march<S0, SN, SH, true, false>);
+  kern<<<grid, 32 * MW, 0, st>>>(bands, approx, Oy, Ox, Oz, o, fb, ty, lo, len, seg);
   return cudaGetLastError();
 }
 
@@ -851,68 +748,25 @@ static size_t synthesis_smem(int reach) {
   return (size_t)(8 * NQ * NQ + 4 * NQ * TP + 2 * TP * TP) * sizeof(float);
 }
 
-// R when every spatial filter has exactly the taps 0..R and every slot filter
-// the taps 0 and 1, else -1
-static int dense_reach(const WaveletBank& bk) {
-  const int R = bk.xy.a[0].n - 1;
-  auto dense = [](const Taps& t, int n) {
-    if (t.n != n) return false;
-    for (int u = 0; u < n; ++u)
-      if (t.k[u] != u) return false;
-    return true;
-  };
-  for (int f = 0; f < 2; ++f)
-    if (!dense(bk.xy.a[f], R + 1) || !dense(bk.xy.s[f], R + 1) || !dense(bk.z.a[f], 2) || !dense(bk.z.s[f], 2))
-      return -1;
-  return R;
-}
-
-// analysis (AN) or synthesis of a dense bank of reach R; the synthesis tile
-// grid is the generic kernel's, the analysis tiles DENSE_TQ coefficients wide
-constexpr int DENSE_TQ = 16;
-template <bool AN, int R>
-static cudaError_t launch_dense(const float* in, const float* approx, int Ly, int Lx, int Lz, int shift, float* out,
-                                const SynthOut& o, const WaveletBank& bk, const LevelBands& th, cudaStream_t st,
-                                const ColRange& cols) {
-  if (AN) {
-    constexpr int T = DENSE_TQ, NY = 2 * T + R;
-    const size_t sm = (size_t)(2 * NY * NY + 4 * T * NY) * sizeof(float);
-    cudaError_t e =
-        cudaFuncSetAttribute(k_wav_analysis_dense<R, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    int t0, nt;
-    tile_span(cols, Lx / 2, T, t0, nt);
-    if (nt == 0) return cudaSuccess;
-    dim3 grid((Ly / 2 + T - 1) / T, nt, Lz / 2);
-    k_wav_analysis_dense<R, T><<<grid, 256, sm, st>>>(in, Ly, Lx, Lz, shift, out, bk, th, t0);
-  } else {
-    const size_t sm = synthesis_smem(R);
-    cudaError_t e = cudaFuncSetAttribute(k_wav_synthesis_dense<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    int t0, nt;
-    tile_span(cols, Lx, TP, t0, nt);
-    if (nt == 0) return cudaSuccess;
-    dim3 grid((Ly + TP - 1) / TP, nt, Lz / 2);
-    k_wav_synthesis_dense<R><<<grid, 256, sm, st>>>(in, approx, Ly, Lx, Lz, o, bk, t0);
-  }
-  return cudaGetLastError();
+// The compile-time kernels take every size of at least the filter length (the
+// generic ones drop taps past the end of a shorter axis).
+static bool march_fits(int kind, int Ly, int Lx, int Lz) {
+  const int W = kind == 1 ? 10 : kind == 2 ? 2 : 8;
+  return kind && Ly >= W && Lx >= W && Lz >= 2 && Ly % 2 == 0 && Lx % 2 == 0 && Lz % 2 == 0;
 }
 
 cudaError_t launch_wav_analysis(const float* in, int Ly, int Lx, int Lz, int shift, float* out,
                                 const WaveletBank& bk, const LevelBands& th, cudaStream_t st,
                                 const ColRange& qcols) {
   const int kind = fast_kind(bk);
-  // the fast kernel wraps each halo coordinate at most once
-  if (kind && Ly > 2 * TQ + 16 && Lx > 2 * TQ + 16 && Lz >= 2) {
+  if (march_fits(kind, Ly, Lx, Lz)) {
     const FastBank fb = fast_bank(bk);
-    if (kind == 1) return launch_analysis_fast<10, 4>(in, Ly, Lx, Lz, shift, out, fb, th, st, qcols);
-    return launch_analysis_fast<2, 0>(in, Ly, Lx, Lz, shift, out, fb, th, st, qcols);
+    const int O = Lx / 2, lo = qcols.all(O) ? 0 : pmod(qcols.lo, O), len = qcols.all(O) ? O : qcols.len;
+    if (len == 0) return cudaSuccess;
+    if (kind == 1) return launch_analysis_march<10, 4, 2>(in, Ly, Lx, Lz, shift, out, fb, th, st, lo, len);
+    if (kind == 2) return launch_analysis_march<2, 0, 2>(in, Ly, Lx, Lz, shift, out, fb, th, st, lo, len);
+    return launch_analysis_march<8, 0, 8>(in, Ly, Lx, Lz, shift, out, fb, th, st, lo, len);
   }
-  // dense sym4 x Haar bank: one wrap of every index is enough when the level
-  // exceeds a tile plus the filter reach and the shift is below every size
-  if (dense_reach(bk) == 7 && shift >= 0 && Ly >= 2 * DENSE_TQ + 7 + shift && Lx >= 2 * DENSE_TQ + 7 + shift &&
-      Lz >= 2 && shift + 1 <= Lz)
-    return launch_dense<true, 7>(in, nullptr, Ly, Lx, Lz, shift, out, SynthOut{}, bk, th, st, qcols);
   const size_t sm = analysis_smem(bk.reach_a);
   cudaError_t e = cudaFuncSetAttribute(k_wav_analysis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
@@ -928,15 +782,17 @@ cudaError_t launch_wav_synthesis(const float* bands, const float* approx, int Oy
                                  const SynthOut& o, const WaveletBank& bk, cudaStream_t st,
                                  const ColRange& cols) {
   const int kind = fast_kind(bk);
-  // coefficient tiles of 37 per axis must wrap at most once; shifts below the size
-  if (kind && Oy >= 128 && Ox >= 128 && Oz >= 2 && o.shift >= 0 && o.shift < Oy && o.shift < Ox) {
+  if (march_fits(kind, Oy, Ox, Oz)) {
     const FastBank fb = fast_bank(bk);
-    if (kind == 1) return launch_synthesis_fast<4, 10>(bands, approx, Oy, Ox, Oz, o, fb, st, cols);
-    return launch_synthesis_fast<0, 2>(bands, approx, Oy, Ox, Oz, o, fb, st, cols);
+    // whole column pairs: the ones that hold the window's columns
+    const int I = Ox / 2, first = pmod(cols.lo, Ox) / 2;
+    const int pairs = cols.all(Ox) ? I : cols.len == 0 ? 0 : (pmod(cols.lo, Ox) + cols.len - 1) / 2 - first + 1;
+    const int lo = pairs >= I ? 0 : first, len = pairs >= I ? I : pairs;
+    if (len == 0) return cudaSuccess;
+    if (kind == 1) return launch_synthesis_march<4, 2, 10>(bands, approx, Oy, Ox, Oz, o, fb, st, lo, len);
+    if (kind == 2) return launch_synthesis_march<0, 2, 2>(bands, approx, Oy, Ox, Oz, o, fb, st, lo, len);
+    return launch_synthesis_march<0, 8, 8>(bands, approx, Oy, Ox, Oz, o, fb, st, lo, len);
   }
-  if (dense_reach(bk) == 7 && Oy >= 2 * TP + 8 && Ox >= 2 * TP + 8 && Oz >= 2 && o.shift >= 0 && o.shift < Oy &&
-      o.shift < Ox && o.shift < Oz)
-    return launch_dense<false, 7>(bands, approx, Oy, Ox, Oz, 0, nullptr, o, bk, LevelBands{}, st, cols);
   const size_t sm = synthesis_smem(bk.reach_s);
   cudaError_t e = cudaFuncSetAttribute(k_wav_synthesis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
