@@ -278,6 +278,223 @@ __global__ void __launch_bounds__(128) k_wiener(WienerArgs A) {
   }
 }
 
+// ---- patch 8, groups of 8 or 16 -----------------------------------------------------
+//
+// The kernel above keeps the shared-memory pipe busy for about 1340 cycles per
+// group of 16, its time: in the first product of each DCT the eight lanes of a
+// page all read the whole page (768 cycles of 16-byte reads).  Here each
+// product is made by the lane that has its vector: lane (page, column) makes a
+// column of T X from the column it reads, lane (page, row) a row of (T X) T' from the row, with
+// T's entries as constant operands; between the two the page passes through shared
+// memory once (64 + 64 values instead of 512).  The inverse goes rows first, then
+// columns, so an output column leaves as two 16-byte stores.  The gains stay
+// in registers: a lane's coefficients are exactly the ones it adds to n2.
+// Every value is the same operation in the same order as above.
+//   Element (r, c) of a page sits at 8 c + (r ^ (c & 4)): columns 4 .. 7 have their
+// halves exchanged, which puts the 16-byte column reads of a page on distinct
+// banks; the page pitch of 72 does the same for the rows of four pages.  36 KB and 80
+// registers: six CTAs per SM (five 1.35 ms, four 1.50 ms at 4096^2).
+//   4096^2 at stride 7 1.60 -> 1.28 ms, 1024^2 dense 1.06 -> 0.86 ms (two spins); now at 84 % of
+// the shared-memory pipe (326 of 843 wavefronts per group are the gather: four
+// lines per 4-byte asynchronous copy) and 81 % of the issue slots (3.5 k instructions).
+template <int K>
+struct Wie8 {
+  static constexpr int PG = 72, BUF = K * PG;
+  static constexpr size_t BYTES = (size_t)4 * 2 * BUF * sizeof(float);
+};
+
+template <int K>
+__global__ void __launch_bounds__(128, 6) k_wiener_8(WienerArgs A) {
+  constexpr int D = 8, DD = 64, PG = Wie8<K>::PG, BUF = Wie8<K>::BUF, GS = DD * K;
+  extern __shared__ __align__(16) float smw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = window_group(blockIdx.x * 4 + warp, A.g0, A.gn, A.M * A.N);
+  if (g < 0) return;
+  float* b1 = smw + warp * 2 * BUF;  // pilot group, later the aggregation weights
+  float* b2 = b1 + BUF;               // noisy group
+  const float cc = 0.70710678118654752440f;
+  const int r = lane % D, kq = lane / D;  // row or column of a page, page of a round of four
+  const int p0 = lane, p1 = 32 + (lane ^ 4);  // places of the lane's elements (and coefficients) lane, lane + 32
+
+  // ---- load the two groups -----------------------------------------------
+  if (A.padP) {
+    const int i = g % A.M, j = g / A.M;
+    unsigned mo = 0;  // lane k: offset of match k in the search image
+    if (lane < K) {
+      int e = (int)A.S[(size_t)g * K + lane] - 1;
+      if ((unsigned)e >= (unsigned)(A.d2 * A.d2)) e = (A.d2 / 2) * (A.d2 + 1);  // never read outside the window
+      const int mb = e / A.d2;
+      mo = (unsigned)(e - mb * A.d2) + (unsigned)mb * (unsigned)A.P;
+    }
+    // the lane's elements of a page: (r, kq) and (r, kq + 4)
+    const size_t base = (size_t)(i * A.s + r) + (size_t)(j * A.s + kq) * A.P;
+    const float* sp0 = A.padP + base;
+    const float* sn0 = A.padN + base;
+    const float* sp1 = sp0 + (size_t)4 * A.P;
+    const float* sn1 = sn0 + (size_t)4 * A.P;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const unsigned o = __shfl_sync(0xffffffffu, mo, k);
+      cp_async4(b1 + k * PG + p0, sp0 + o);
+      cp_async4(b1 + k * PG + p1, sp1 + o);
+      cp_async4(b2 + k * PG + p0, sn0 + o);
+      cp_async4(b2 + k * PG + p1, sn1 + o);
+    }
+    cp_async_wait_all();
+  } else {
+    const float* v1 = A.V1 + (size_t)g * GS;
+    const float* v2 = A.V2 + (size_t)g * GS;
+    for (int k = 0; k < K; ++k) {
+      b1[k * PG + p0] = v1[k * DD + lane];
+      b1[k * PG + p1] = v1[k * DD + lane + 32];
+      b2[k * PG + p0] = v2[k * DD + lane];
+      b2[k * PG + p1] = v2[k * DD + lane + 32];
+    }
+  }
+  __syncwarp();
+
+  // ---- forward DCT of each page, in place: P = T X by columns, then P T' by rows,
+  // each sum a serial fmaf chain from 0 in ascending index
+  const int h0 = r & 4;  // column r's first half starts at 8 r + h0
+#pragma unroll 1
+  for (int k0 = 0; k0 < 2 * K; k0 += 4) {  // pages of b1, then of b2 (contiguous)
+    float* x = b1 + (k0 + kq) * PG;
+    {
+      const float4 lo = *reinterpret_cast<const float4*>(x + D * r + h0);
+      const float4 hi = *reinterpret_cast<const float4*>(x + D * r + (h0 ^ 4));
+      const float c[D] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      float P[D];
+#pragma unroll
+      for (int q = 0; q < D; ++q) {
+        float acc = 0.f;
+#pragma unroll
+        for (int jj = 0; jj < D; ++jj) acc = fmaf(A.T[q + jj * D], c[jj], acc);
+        P[q] = acc;
+      }
+      *reinterpret_cast<float4*>(x + D * r + h0) = make_float4(P[0], P[1], P[2], P[3]);
+      *reinterpret_cast<float4*>(x + D * r + (h0 ^ 4)) = make_float4(P[4], P[5], P[6], P[7]);
+    }
+    __syncwarp();
+    {
+      float P[D];
+#pragma unroll
+      for (int n = 0; n < D; ++n) P[n] = x[D * n + (r ^ (n & 4))];
+#pragma unroll
+      for (int l = 0; l < D; ++l) {
+        float acc = 0.f;
+#pragma unroll
+        for (int n = 0; n < D; ++n) acc = fmaf(P[n], A.T[l + n * D], acc);
+        x[D * l + (r ^ (l & 4))] = acc;
+      }
+    }
+  }
+  __syncwarp();
+
+  // ---- Haar along slots, Wiener gain, inverse Haar: lane has coefficients lane
+  // and lane + 32 (places p0, p1), read and written by it alone
+  float f0[K];
+  float s = 0.f;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int e = lane + 32 * u, p = u ? p1 : p0;
+    float v1[K], v2[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      v1[k] = b1[k * PG + p];
+      v2[k] = b2[k * PG + p];
+    }
+    haar_dec<K>(v1, cc);
+    haar_dec<K>(v2, cc);
+    const float sg = A.s2[e];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const float w = v1[k] * v1[k];
+      float f = w / (w + sg);
+      if (e == 0 && k >= 14) f = 1.f;
+      v2[k] = v2[k] * f;
+      // n2's partial sum of this lane: slot by slot, coefficient lane, then lane + 32
+      if (u == 0) {
+        f0[k] = f;
+      } else {
+        s = s + f0[k] * f0[k];
+        s = s + f * f;
+      }
+    }
+    haar_rec<K>(v2, cc);
+#pragma unroll
+    for (int k = 0; k < K; ++k) b2[k * PG + p] = v2[k];
+  }
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, off);
+  // weight = w / norm(col(filt))^2 (denoiseAndAggregateWieFast.m:81), one
+  // division per window position, shared by the K blocks of the group
+  const float nr = sqrtf(s), n2 = nr * nr;
+  if (lane == 0) A.n2[g] = n2;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int e = lane + 32 * u;
+    const float wv = A.win[e] / n2;
+    b1[e] = wv;  // every lane's gains, made from b1, are in s
+    A.wt[(size_t)g * DD + e] = wv;
+  }
+  __syncwarp();
+
+  // ---- inverse DCT: P = Y Ti' by rows, then Ti P by columns to global memory
+  float wc[D];
+#pragma unroll
+  for (int q = 0; q < D; q += 4) {
+    const float4 w = *reinterpret_cast<const float4*>(b1 + D * r + q);
+    wc[q] = w.x; wc[q + 1] = w.y; wc[q + 2] = w.z; wc[q + 3] = w.w;
+  }
+  float* og = A.out + (size_t)g * GS;
+#pragma unroll 1
+  for (int k0 = 0; k0 < K; k0 += 4) {
+    float* y = b2 + (k0 + kq) * PG;
+    {
+      float Y[D];
+#pragma unroll
+      for (int n = 0; n < D; ++n) Y[n] = y[D * n + (r ^ (n & 4))];
+#pragma unroll
+      for (int l = 0; l < D; ++l) {
+        float acc = 0.f;
+#pragma unroll
+        for (int n = 0; n < D; ++n) acc = fmaf(Y[n], A.Ti[l + n * D], acc);
+        y[D * l + (r ^ (l & 4))] = acc;
+      }
+    }
+    __syncwarp();
+    {
+      const float4 lo = *reinterpret_cast<const float4*>(y + D * r + h0);
+      const float4 hi = *reinterpret_cast<const float4*>(y + D * r + (h0 ^ 4));
+      const float c[D] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      float z[D];
+#pragma unroll
+      for (int q = 0; q < D; ++q) {
+        float acc = 0.f;
+#pragma unroll
+        for (int jj = 0; jj < D; ++jj) acc = fmaf(A.Ti[q + jj * D], c[jj], acc);
+        float v = acc > 0.f ? acc : 0.f;
+        if (A.clamp_one && v > 1.f) v = 1.f;
+        z[q] = wc[q] * v;  // weight.*blocks(:,:,i) (:84-90)
+      }
+      float4* d = reinterpret_cast<float4*>(og + (k0 + kq) * DD + D * r);
+      d[0] = make_float4(z[0], z[1], z[2], z[3]);
+      d[1] = make_float4(z[4], z[5], z[6], z[7]);
+    }
+  }
+}
+
+template <int K>
+static cudaError_t launch_wiener_8(const WienerArgs& A, cudaStream_t st) {
+  const size_t sm = Wie8<K>::BYTES;
+  cudaError_t e = cudaFuncSetAttribute(k_wiener_8<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  const int G = A.gn > 0 ? A.gn : A.M * A.N;
+  if (A.gn < 0) return cudaSuccess;  // an empty window
+  k_wiener_8<K><<<(G + 3) / 4, 128, sm, st>>>(A);
+  return cudaGetLastError();
+}
+
 bool wiener_supported(int d, int K) { return (d == 4 || d == 8 || d == 16) && (K == 8 || K == 16 || K == 32); }
 
 template <int D, int K>
@@ -293,9 +510,11 @@ static cudaError_t launch_wiener_t(const WienerArgs& A, cudaStream_t st) {
 
 cudaError_t launch_wiener(int d, const WienerArgs& A, cudaStream_t st) {
   if (A.padP && (A.s < 1 || A.s > d)) return cudaErrorInvalidValue;
+  if (d == 8 && A.K == 16) return launch_wiener_8<16>(A, st);
+  if (d == 8 && A.K == 8) return launch_wiener_8<8>(A, st);
 #define GBM3D_WIE_CASE(DD, KK) \
   if (d == DD && A.K == KK) return launch_wiener_t<DD, KK>(A, st);
-  GBM3D_WIE_CASE(8, 16) GBM3D_WIE_CASE(8, 8) GBM3D_WIE_CASE(8, 32)
+  GBM3D_WIE_CASE(8, 32)
   GBM3D_WIE_CASE(4, 16) GBM3D_WIE_CASE(4, 8) GBM3D_WIE_CASE(4, 32)
   GBM3D_WIE_CASE(16, 16) GBM3D_WIE_CASE(16, 8)
 #undef GBM3D_WIE_CASE
