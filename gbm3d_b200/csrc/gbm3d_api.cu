@@ -354,14 +354,6 @@ __global__ void k_accum2(const float* __restrict__ u, const float* __restrict__ 
   wa[o] = first ? y : wa[o] + y;
 }
 
-__global__ void k_accum(const float* __restrict__ v, int Mp, int Np, int s, double* __restrict__ acc, int first) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
-  if (r >= Mp || c >= Np) return;
-  const double x = (double)v[pmod(r + s, Mp) + (size_t)pmod(c + s, Np) * Mp];
-  const size_t o = r + (size_t)c * Mp;
-  acc[o] = first ? x : acc[o] + x;
-}
-
 __global__ void k_shift_copy(const float* __restrict__ v, int Mp, int Np, int s, float* __restrict__ out) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
   if (r >= Mp || c >= Np) return;
@@ -1694,9 +1686,7 @@ void pipeline_rgb(gbm3d_ctx* c, const double* const* dI, int m, int n, double si
       std::vector<double> tau(tau1);
       for (auto& t : tau) t *= csig[ch];
       run_ht(c, vol, S1, cnt1, M1, N1, d, d2, K, o->levels, o->cycleSpin, tau.data(), bk, Us, Ws, o->filtType, st1);
-      k_accum<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Mp, Np, s, Ua[ch], ii == 0);
-      launched(c, cudaGetLastError(), "accum");
-      k_accum<<<grid2(Mp, Np), 256, 0, c->st>>>(Ws, Mp, Np, s, Wa[ch], ii == 0);
+      k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua[ch], Wa[ch], ii == 0);
       launched(c, cudaGetLastError(), "accum");
     }
   }
@@ -1730,9 +1720,7 @@ void pipeline_rgb(gbm3d_ctx* c, const double* const* dI, int m, int n, double si
       A.s = st2;
       fill_wiener_consts(A, dw, &csig[ch], 0, 0);
       run_wiener_agg(c, A, dw, d2, Us, Ws);
-      k_accum<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Mp, Np, s, Ua[ch], ii == 0);
-      launched(c, cudaGetLastError(), "accum");
-      k_accum<<<grid2(Mp, Np), 256, 0, c->st>>>(Ws, Mp, Np, s, Wa[ch], ii == 0);
+      k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua[ch], Wa[ch], ii == 0);
       launched(c, cudaGetLastError(), "accum");
     }
   }

@@ -230,28 +230,42 @@ cudaError_t launch_match(int d, int d2, const MatchArgs& A, cudaStream_t st) {
 // Gather the blocks a match set selects from another image's search image:
 // the colour form matches on luma and filters every channel with those sets.
 // vol is tile-space (vm = M d rows), block (i, j) slot k at rows i d, cols j d.
-__global__ void k_gather_volume(const float* __restrict__ pad, int P, int M, int N, int s, int d, int d2, int K,
-                                const uint32_t* __restrict__ S, const int32_t* __restrict__ cnt,
-                                float* __restrict__ vol, int vm, int vn) {
-  const size_t total = (size_t)M * N * K * d * d;
-  const int h = d2 / 2;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    const int r = (int)(t % d), c = (int)((t / d) % d);
-    const size_t gk = t / ((size_t)d * d);
-    const int k = (int)(gk % K);
-    const size_t g = gk / K;
-    const int i = (int)(g % M), j = (int)(g / M);
-    int e = (int)S[g * K + k] - 1;
-    if ((cnt && k >= cnt[g]) || (unsigned)e >= (unsigned)(d2 * d2)) e = h + h * d2;
-    const int a = e % d2, b = e / d2;
-    vol[(size_t)(i * d + r) + (size_t)vm * (j * d + c) + (size_t)vm * vn * k] =
-        pad[(size_t)(i * s + a + r) + (size_t)(j * s + b + c) * P];
+// A thread per row and column, rows along the threads, all slots in turn: stores
+// are whole lines and d rows share a match index.  The flat version of it
+// (divisions of 64-bit indices, stores in d-element pieces) took 162 us for
+// 1024^2 x 16; this 33.
+template <int D>
+__global__ void __launch_bounds__(256) k_gather_volume(const float* __restrict__ pad, int P, int M, int s, int d2,
+                                                       int K, const uint32_t* __restrict__ S,
+                                                       const int32_t* __restrict__ cnt, float* __restrict__ vol) {
+  const int y = blockIdx.x * 256 + threadIdx.x, x = blockIdx.y, vm = M * D;
+  if (y >= vm) return;
+  const int i = y / D, r = y % D, j = x / D, c = x % D, h = d2 / 2;
+  const size_t g = i + (size_t)M * j;
+  const int nm = cnt ? __ldg(cnt + g) : K;
+  const uint32_t* Sg = S + g * K;
+  const float* src = pad + (size_t)(i * s + r) + (size_t)(j * s + c) * P;
+  float* dst = vol + y + (size_t)vm * x;
+  const size_t slot = (size_t)vm * gridDim.y;
+#pragma unroll 8
+  for (int k = 0; k < K; ++k) {
+    int e = (int)__ldg(Sg + k) - 1;
+    if (k >= nm || (unsigned)e >= (unsigned)(d2 * d2)) e = h + h * d2;
+    const int b = d2 == 32 ? e >> 5 : e / d2, a = e - b * d2;
+    dst[slot * k] = __ldg(src + a + (size_t)b * P);
   }
 }
 
 cudaError_t launch_gather_volume(const float* pad, int P, int M, int N, int s, int d, int d2, int K, const uint32_t* S,
                                  const int32_t* cnt, float* vol, cudaStream_t st) {
-  k_gather_volume<<<1184, 256, 0, st>>>(pad, P, M, N, s, d, d2, K, S, cnt, vol, M * d, N * d);
+  const dim3 grid((M * d + 255) / 256, N * d);
+  if (N * d > 65535) return cudaErrorInvalidValue;
+  switch (d) {
+    case 8: k_gather_volume<8><<<grid, 256, 0, st>>>(pad, P, M, s, d2, K, S, cnt, vol); break;
+    case 16: k_gather_volume<16><<<grid, 256, 0, st>>>(pad, P, M, s, d2, K, S, cnt, vol); break;
+    case 32: k_gather_volume<32><<<grid, 256, 0, st>>>(pad, P, M, s, d2, K, S, cnt, vol); break;
+    default: return cudaErrorInvalidValue;
+  }
   return cudaGetLastError();
 }
 

@@ -647,54 +647,67 @@ static cudaError_t launch_synthesis_march(const float* bands, const float* appro
   return cudaGetLastError();
 }
 
-// Compile-time block size version of k_ht_weights.  The group is streamed one
-// slot at a time through a shared-memory slice (read once, coalesced).  Every
-// difference array is slot-major, so walking the slots in order keeps each
-// lane's elements (e = lane + 32 t of each array) in increasing e: the sums
-// are the same fixed-order reductions as the generic kernel and the oracle.
-// GM: V is group-major (SynthOut), else image-shaped m x n x K.
+// k_ht_weights for patches 16 and 32, one CTA per group: the group's slots are staged
+// in shared memory ([k][c][r], 16-byte copies), then one warp adds each of the
+// three terms, so the terms' serial chains run side by side.  Each is the
+// same fixed-order reduction as in the generic kernel and the oracle: lane l adds
+// the elements l, l + 32, ... of the column-major difference array (indices advanced by 32
+// with carries), then an xor butterfly.  One warp per group, slot by slot, took
+// 44 us for the 48 groups of 128 x 96 (here 8) and 82 us for a 720p frame's 920
+// (here 51: 64 KB of slots allow three CTAs per SM, and each chain has 464 adds).
+// GM: V is group-major (SynthOut), else image-shaped m x n x K (m a multiple of D).
 template <int D, bool GM>
-__global__ void __launch_bounds__(128) k_ht_weights_t(const float* __restrict__ V, int m, int n, int M, int N,
-                                                      int K, const int32_t* __restrict__ cnt,
-                                                      float* __restrict__ wgt, int g0, int gn) {
-  constexpr int DM = D - 3, SL = D * D, SX = D * DM;  // slice size, per-slot elements of the x/y terms
-  __shared__ float sl[4][2][SL];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = window_group(blockIdx.x * 4 + warp, g0, gn, M * N);
+__global__ void __launch_bounds__(96) k_ht_weights_cta(const float* __restrict__ V, int m, int n, int M, int N, int K,
+                                                       const int32_t* __restrict__ cnt, float* __restrict__ wgt,
+                                                       int g0, int gn) {
+  constexpr int DM = D - 3, SL = D * D;
+  extern __shared__ __align__(16) float sg[];
+  __shared__ float sum[3];
+  const int term = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = window_group(blockIdx.x, g0, gn, M * N);
   if (g < 0) return;
   const int i = g % M, j = g / M;
   const int nm = cnt ? cnt[g] : K;
-  const size_t sz = GM ? (size_t)SL : (size_t)m * n, cs = GM ? (size_t)D : (size_t)m;
+  const size_t ks = GM ? (size_t)SL : (size_t)m * n, cs = GM ? (size_t)D : (size_t)m;
   const float* base = GM ? V + (size_t)g * K * SL : V + (size_t)i * D + (size_t)j * D * m;
-  float tx = 0.f, ty = 0.f, tz = 0.f;
-  for (int k = 0; k < nm; ++k) {
-    float* cur = sl[warp][k & 1];
-    const float* prv = sl[warp][(k & 1) ^ 1];
-    for (int t = lane; t < SL; t += 32) cur[t] = __ldg(base + (t % D) + (size_t)(t / D) * cs + sz * k);
-    __syncwarp();
-    // x term: element r + D (c + DM k); this lane's first element of slot k
-    for (int e = ((lane - k * SX) % 32 + 32) % 32; e < SX; e += 32) {
-      const int r = e % D, c = e / D;
-      const float* p = cur + r + c * D;
-      tx = tx + fabsf(d3(p[0], p[D], p[2 * D], p[3 * D]));
-    }
-    // y term: element r + DM (c + D k)
-    for (int e = ((lane - k * SX) % 32 + 32) % 32; e < SX; e += 32) {
-      const int r = e % DM, c = e / DM;
-      const float* p = cur + r + c * D;
-      ty = ty + fabsf(d3(p[0], p[1], p[2], p[3]));
-    }
-    // slot term: element r + D (c + D (k-1)) for the pair (k-1, k)
-    if (k > 0)
-      for (int e = ((lane - (k - 1) * SL) % 32 + 32) % 32; e < SL; e += 32) tz = tz + fabsf(cur[e] - prv[e]);
-    __syncwarp();
+  for (int t = threadIdx.x; t < nm * (SL / 4); t += 96) {
+    const int k = t / (SL / 4), c = t % (SL / 4) / (D / 4), r = 4 * (t % (D / 4));
+    cp_async16(sg + 4 * t, base + ks * k + cs * c + r);
   }
-  tx = warp_sum(tx);
-  ty = warp_sum(ty);
-  tz = warp_sum(tz);
-  if (lane == 0) {
-    float w = tx * 0.25f + ty * 0.25f;
-    w = w + tz;
+  cp_async_wait_all();
+  __syncthreads();
+  float acc = 0.f;
+  const int nx = D * DM * nm;
+  if (term == 0) {  // x: element r + D (c + DM k)
+    int c = lane / D;
+    const float* q = sg + lane;  // element (r, c, k)
+#pragma unroll 8
+    for (int e = lane; e < nx; e += 32) {
+      acc = acc + fabsf(d3(q[0], q[D], q[2 * D], q[3 * D]));
+      q += 32;
+      c += 32 / D;
+      if (c >= DM) c -= DM, q += 3 * D;
+    }
+  } else if (term == 1) {  // y: element r + DM (c + D k)
+    int r = lane % DM;
+    const float* q = sg + (lane / DM) * D + r;
+#pragma unroll 8
+    for (int e = lane; e < nx; e += 32) {
+      acc = acc + fabsf(d3(q[0], q[1], q[2], q[3]));
+      q += (32 / DM) * D + 32 % DM;
+      r += 32 % DM;
+      if (r >= DM) r -= DM, q += D - DM;
+    }
+  } else {  // slots: element r + D (c + D k) of the pair (k, k + 1)
+#pragma unroll 8
+    for (int e = lane; e < (nm - 1) * SL; e += 32) acc = acc + fabsf(sg[e + SL] - sg[e]);
+  }
+  acc = warp_sum(acc);
+  if (lane == 0) sum[term] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float w = sum[0] * 0.25f + sum[1] * 0.25f;
+    w = w + sum[2];
     wgt[g] = 1.f / (w + 2.220446049250313e-16f);
   }
 }
@@ -827,7 +840,20 @@ __global__ void __launch_bounds__(128) k_ht_weights_8(const float* __restrict__ 
   const float* p0 = GM ? V + (size_t)g * K * SL + lane
                        : V + (size_t)i * D + (size_t)(j * D + (lane >> 3)) * m + (lane & 7);
   const float* p1 = p0 + (GM ? (size_t)32 : (size_t)4 * m);
-  // slots in batches of 4: eight independent loads in flight per lane
+  // slots in batches of 4: eight independent loads in flight per lane.  The slot
+  // term's elements lane and lane + 32 of a pair (k - 1, k) are the lane's own values.
+  float tx = 0.f, ty = 0.f, tz = 0.f;
+  float pa = 0.f, pb = 0.f;
+  auto slot = [&](int k, float a, float b) {
+    sg[k * SL + lane] = a;
+    sg[k * SL + 32 + lane] = b;
+    if (k > 0) {
+      tz = tz + fabsf(a - pa);
+      tz = tz + fabsf(b - pb);
+    }
+    pa = a;
+    pb = b;
+  };
   int k = 0;
   for (; k + 4 <= nm; k += 4) {
     float a[4], b[4];
@@ -837,17 +863,10 @@ __global__ void __launch_bounds__(128) k_ht_weights_8(const float* __restrict__ 
       b[u] = __ldg(p1 + sz * (k + u));
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      sg[(k + u) * SL + lane] = a[u];
-      sg[(k + u) * SL + 32 + lane] = b[u];
-    }
+    for (int u = 0; u < 4; ++u) slot(k + u, a[u], b[u]);
   }
-  for (; k < nm; ++k) {
-    sg[k * SL + lane] = __ldg(p0 + sz * k);
-    sg[k * SL + 32 + lane] = __ldg(p1 + sz * k);
-  }
+  for (; k < nm; ++k) slot(k, __ldg(p0 + sz * k), __ldg(p1 + sz * k));
   __syncwarp();
-  float tx = 0.f, ty = 0.f, tz = 0.f;
   // x term: element r + D (c + DM k) -> V(r, c .. c+3, k) at r + D c + SL k = e + (SL - SX) k
   for (int e = lane; e < nm * SX; e += 32) {
     const int k = e / SX;
@@ -860,8 +879,6 @@ __global__ void __launch_bounds__(128) k_ht_weights_8(const float* __restrict__ 
     const float* q = sg + k * SL + c * D + r;
     ty = ty + fabsf(d3(q[0], q[1], q[2], q[3]));
   }
-  // slot term: element r + D (c + D k) of the pair (k, k+1)
-  for (int e = lane; e < (nm - 1) * SL; e += 32) tz = tz + fabsf(sg[e + SL] - sg[e]);
   tx = warp_sum(tx);
   ty = warp_sum(ty);
   tz = warp_sum(tz);
@@ -885,13 +902,14 @@ cudaError_t launch_ht_weights(const float* Vavg, int m, int n, int M, int N, int
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
     if (e != cudaSuccess) return e;
     kern<<<(G + 3) / 4, 128, smb, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
-  } else if (d == 16) {
-    auto kern = group_major ? k_ht_weights_t<16, true> : k_ht_weights_t<16, false>;
-    kern<<<(G + 3) / 4, 128, 0, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
+  } else if (d == 16 || (d == 32 && !group_major)) {
+    auto kern = d == 32 ? k_ht_weights_cta<32, false> : group_major ? k_ht_weights_cta<16, true> : k_ht_weights_cta<16, false>;
+    const size_t smb = (size_t)K * d * d * sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
+    if (e != cudaSuccess) return e;
+    kern<<<G, 96, smb, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
   } else if (group_major) {
     return cudaErrorInvalidValue;
-  } else if (d == 32) {
-    k_ht_weights_t<32, false><<<(G + 3) / 4, 128, 0, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
   } else {
     k_ht_weights<<<(G + 3) / 4, 128, 0, st>>>(Vavg, m, n, M, N, d, K, cnt, wgt, g0, gn);
   }
