@@ -1768,6 +1768,7 @@ void video_window(gbm3d_ctx* c, float* const* pads, int P, int m, int n, int F, 
   A.n = n;
   A.S = S;
   A.volume = vol;
+  A.redo = buf<int>(c, "v.redo", (size_t)M * N);
   {
     StageTimer t(c, 1);
     launched(c, launch_match_video(d, A, c->st), "match_video");
@@ -1924,6 +1925,7 @@ int gbm3d_matchBlocksV(gbm3d_ctx* c, const double* I, int m, int n, int frames, 
     A.n = n;
     A.S = dS;
     A.volume = dV;
+    A.redo = buf<int>(c, "v.redo", (size_t)M * N);
     launched(c, launch_match_video(d, A, c->st), "match_video");
     ck(c, cudaMemcpyAsync(S, dS, (size_t)K * M * N * 4, cudaMemcpyDeviceToHost, c->st), "D2H");
     if (Volume) ck(c, cudaMemcpyAsync(Volume, dV, px * K * 4, cudaMemcpyDeviceToHost, c->st), "D2H");

@@ -229,8 +229,15 @@ struct VideoMatchArgs {
   int m, n;               // frame size (volume rows / columns)
   uint32_t* S;            // K x M x N, 1-based index a + b d + f d^2 into the d x d x F window
   float* volume;          // m x n x K
+  // one int per reference (may be null): with it, patch 32 runs the bounded matcher
+  // first, and the direct one only on the references that it marks here
+  int* redo;
 };
 bool video_match_supported(int d, int F, int K);
+// Patch 32 (video_bound.cu): tensor-core distances bound the candidates, the exact
+// FP32 SSD ranks them; the direct matcher's sets.
+bool video_bound_supported(int d, const VideoMatchArgs& A);
+cudaError_t launch_match_video_bound(const VideoMatchArgs& A, cudaStream_t st);
 cudaError_t launch_match_video(int d, const VideoMatchArgs& A, cudaStream_t st);
 struct VideoAggArgs {
   const uint32_t* S;

@@ -15,20 +15,9 @@
 // consumed by the warp that made them; the tcgen05 version (match_tc.cu) needs
 // tile-wide barriers and TMEM round trips around its selection and is slower.
 //
-// The bound.  All values are centred by a number m0 common to the CTA and
-// rounded to f16: x16, w16.  With r = ||x - w|| (the true distance) and
-// r16 = ||x16 - w16||, |r - r16| <= u (||x'|| + ||w'||) + 2 eta
-// <= u (2 ||x'|| + r) + 2 eta, u = 2^-11 the f16 rounding unit, eta = 8 2^-25
-// its subnormal part: the error is that of two roundings, not of a product, so
-// it vanishes with the patch's contrast.  The computed squared distance is
-// d = ||x16||^2 - 2 v, v = <x16, w16> - ||w16||^2 / 2 (the norm sums are those of
-// the rounded values), with |d - r16^2| <= kappa (||x16||^2 + ||w16||^2); kappa =
-// 2.2e-5 covers eight MMA steps of nine addends each truncated at 2^-23 of
-// the largest, and the FP32 sums.  From T, a value that at least K candidates'
-// d do not exceed, candidate_threshold() derives theta such that every
-// candidate of the exact top K (in the kernel's own FP32 distances, whose
-// relative error is below 70 2^-24) has d <= theta.  Those are listed and
-// ranked by the exact SSD and index, as the exhaustive matcher ranks.
+// The bound itself, candidate_threshold(), is derived in bound.cuh.  The candidates
+// it leaves are listed and ranked by the exact SSD and index, as the exhaustive
+// matcher ranks.
 //
 // A CTA takes four references of one grid row (i; j .. j + 3): their windows
 // overlap, so the union (39 x (3 s + 39)) is staged by one TMA copy, rounded to
@@ -46,6 +35,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include "bound.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
 #include "match_search.cuh"
@@ -65,47 +55,6 @@ constexpr int LCAND = 128;                                  // candidates a warp
 // 32-bit words of a warp's scratch: the exhaustive search's 224, or 64 (reference
 // block, row-major) + 32 (S) + 2 LCAND (keys and indices)
 constexpr int SCR = 96 + 2 * LCAND;
-
-__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr));
-}
-
-__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                        uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// theta (see the header): T bounds the K-th smallest computed squared distance,
-// nx = ||x16||^2.
-__device__ __forceinline__ float candidate_threshold(float T, float nx) {
-  constexpr float U = 4.8852e-4f;  // 2^-11 (1 + 2^-11)
-  constexpr float ETA2 = 4.8e-7f;  // 2 eta
-  constexpr float KAPPA = 2.2e-5f, GAMMA2 = 1.0e-5f;
-  const float X = sqrtf(nx) * (1.f + 2.f * U) + ETA2;                                // >= ||x'||
-  const float A = sqrtf((fmaxf(T, 0.f) + 3.f * KAPPA * nx) * (1.f + 3.f * KAPPA));   // >= r16 of K candidates
-  const float R = (A + 2.f * U * X + ETA2) * (1.f + 2.f * U) * (1.f + GAMMA2);       // >= r of the exact top K
-  const float R16 = R * (1.f + U) + 2.f * U * X + ETA2;                              // >= their r16
-  return (R16 * R16 * (1.f + 2.f * KAPPA) + 3.f * KAPPA * nx) * (1.f + 1e-6f);       // >= their d
-}
-
-// Descending bitonic sort of one value per lane.
-__device__ __forceinline__ float sort_desc(float v, int lane) {
-#pragma unroll
-  for (int k2 = 2; k2 <= 32; k2 <<= 1)
-#pragma unroll
-    for (int j2 = k2 >> 1; j2 > 0; j2 >>= 1) {
-      const float o = __shfl_xor_sync(0xffffffffu, v, j2);
-      const bool up = ((lane & k2) == 0), lower = ((lane & j2) == 0);
-      v = (lower == up) ? fmaxf(v, o) : fminf(v, o);
-    }
-  return v;
-}
 
 // Groups of the column range [j0, j0 + nj): blockIdx.x = i + M (tile of four columns).
 __global__ void __launch_bounds__(128, 6) k_match_bound(const __grid_constant__ CUtensorMap tmap, MatchArgs A, int j0,
@@ -274,7 +223,7 @@ __global__ void __launch_bounds__(128, 6) k_match_bound(const __grid_constant__ 
 #pragma unroll
     for (int e = 1; e < 32; ++e) m1 = fmaxf(m1, acc[e >> 4][(e >> 2) & 3][e & 3]);
     const float v1 = sort_desc(m1, lane);
-    float th = 0.5f * (nx - candidate_threshold(nx - 2.f * __shfl_sync(FULL, v1, K - 1), nx));
+    float th = 0.5f * (nx - candidate_threshold<Bound8>(nx - 2.f * __shfl_sync(FULL, v1, K - 1), nx));
     uint32_t hits = 0;
 #pragma unroll
     for (int e = 0; e < 32; ++e) hits |= acc[e >> 4][(e >> 2) & 3][e & 3] >= th ? 1u << e : 0u;
@@ -294,7 +243,7 @@ __global__ void __launch_bounds__(128, 6) k_match_bound(const __grid_constant__ 
 #pragma unroll
       for (int q = 16; q >= 1; q >>= 1) best = fmaxf(best, __shfl_xor_sync(FULL, best, q));
       best = fmaxf(best, __shfl_sync(FULL, v1, K - 1));
-      th = 0.5f * (nx - candidate_threshold(nx - 2.f * best, nx));
+      th = 0.5f * (nx - candidate_threshold<Bound8>(nx - 2.f * best, nx));
       hits = 0;
 #pragma unroll
       for (int e = 0; e < 32; ++e) hits |= acc[e >> 4][(e >> 2) & 3][e & 3] >= th ? 1u << e : 0u;

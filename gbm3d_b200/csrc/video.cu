@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(128) k_match_video(VideoMatchArgs A) {
   __shared__ uint32_t sel[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = blockIdx.x, i = g % A.M, j = g / A.M;
+  if (A.redo && !A.redo[g]) return;  // the bounded matcher has done it
   const int ref = (A.F - 1) / 2;
   const int nc = A.F * DD;
   {  // the reference block: offset (d/2, d/2) of the centre frame's window
@@ -180,8 +181,15 @@ bool video_match_supported(int d, int F, int K) {
          (size_t)F * d * d * 8 + (size_t)(4 * d * d + d * d) * 4 <= 200 * 1024;
 }
 
-cudaError_t launch_match_video(int d, const VideoMatchArgs& A, cudaStream_t st) {
+cudaError_t launch_match_video(int d, const VideoMatchArgs& B, cudaStream_t st) {
+  VideoMatchArgs A = B;
   if (!video_match_supported(d, A.F, A.K)) return cudaErrorInvalidValue;
+  if (video_bound_supported(d, A)) {
+    const cudaError_t e = launch_match_video_bound(A, st);
+    if (e != cudaSuccess) return e;
+  } else {
+    A.redo = nullptr;
+  }
   const size_t sm = (size_t)A.F * d * d * 8 + (size_t)(4 * d * d + d * d) * 4;
   const int G = A.M * A.N;
 #define GBM3D_VM_CASE(DD)                                                                                   \

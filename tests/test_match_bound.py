@@ -90,3 +90,20 @@ def test_threshold_keeps_the_exact_top_k(scale, contrast, noise):
         theta = _threshold(np.float32(np.sort(d)[K - 1]), np.float32(nx))
         top = np.argsort(exact, kind="stable")[:K]
         assert np.all(d[top] <= theta)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,m,n,F,K", [
+    ("noisy", 64, 96, 3, 16), ("noisy", 96, 64, 5, 8), ("noisy", 64, 64, 7, 32), ("noisy", 64, 64, 9, 16),
+    ("noisy", 64, 96, 11, 1), ("noisy", 64, 64, 13, 16), ("smooth", 96, 96, 3, 16), ("tiny", 64, 64, 3, 16),
+    ("overflow", 64, 64, 3, 16), ("flat", 64, 96, 3, 16), ("step", 96, 96, 3, 16),
+])
+def test_bounded_video_matching_equals_the_direct_search(gpu, oracle, kind, m, n, F, K):
+    """Patch 32 (csrc/video_bound.cu): windows of 3 to 11 frames, and one beyond."""
+    from gbm3d_b200 import api
+    base = _image(kind, m, n, seed=m + F)
+    I = np.stack([np.roll(base, f, axis=0) + (0 if kind in ("flat", "step") else f * 1e-3 * base) for f in range(F)], axis=2)
+    S, V = api.matchBlocksV(I, 0.1, {"blockSize": 32, "numMax": K, "numMin": K, "nF": F})
+    So, Vo = oracle.matchBlocksV(I, 32, K, prec=32)
+    assert np.array_equal(np.asarray(S), So), f"{int((np.asarray(S) != So).any(axis=0).sum())} match sets differ"
+    assert np.array_equal(V, Vo)
