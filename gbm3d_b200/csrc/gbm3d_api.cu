@@ -534,7 +534,7 @@ struct Spin2Cols {
 
 float* run_wavelet_ht(gbm3d_ctx* c, const float* vol, int m, int n, int K, int levels, int cycleSpin,
                       const double* tau, const WaveletBank& bk, int filtType, const Spin1Cols* w = nullptr,
-                      int gs = 0) {
+                      int gs = 0, bool clamp1 = false) {
   float* vsum = buf<float>(c, "ht.vsum", (size_t)m * n * K);
   if (filtType == 1) {  // medfilt3 instead of the wavelet (denoiseAndAggregateGPU.m:49-52)
     StageTimer tw(c, 2);
@@ -577,6 +577,7 @@ float* run_wavelet_ht(gbm3d_ctx* c, const float* vol, int m, int n, int K, int l
         o.gs = gs;
         o.pow2 = (cycleSpin & (cycleSpin - 1)) == 0;
         o.inv = 1.f / (float)cycleSpin;
+        o.clamp1 = clamp1;
       } else {
         o.out = rec[lv];
         o.shift = 0;
@@ -1752,10 +1753,10 @@ void check_video(gbm3d_ctx* c, const gbm3d_opts* o, int d, int F, int K) {
 }
 
 // matchBlocksV + denoiseAndAggregateV on one window whose F search images are
-// built (pads); U, W: m x n x F double (device).
+// built (pads), its sums added to Y and nn: m x n x F single (device).
 void video_window(gbm3d_ctx* c, float* const* pads, int P, int m, int n, int F, int d, int K, int levels,
-                  int cycleSpin, const double* tau, const WaveletBank& bk, uint32_t* S, float* vol, double* U,
-                  double* W) {
+                  int cycleSpin, const double* tau, const WaveletBank& bk, uint32_t* S, float* vol, float* Y,
+                  float* nn) {
   const int M = m / d, N = n / d;
   VideoMatchArgs A{};
   for (int f = 0; f < F; ++f) A.pads[f] = pads[f];
@@ -1776,8 +1777,7 @@ void video_window(gbm3d_ctx* c, float* const* pads, int P, int m, int n, int F, 
   float* vsum;
   {
     StageTimer t(c, 2);
-    vsum = run_wavelet_ht(c, vol, m, n, K, levels, cycleSpin, tau, bk, 0);
-    launched(c, launch_clamp01(vsum, (size_t)m * n * K, c->st), "clamp");  // Vavg = min(max(.,0),1)
+    vsum = run_wavelet_ht(c, vol, m, n, K, levels, cycleSpin, tau, bk, 0, nullptr, 0, true);  // Vavg = min(max(.,0),1)
   }
   StageTimer t(c, 3);
   float* wgt = buf<float>(c, "v.wgt", (size_t)M * N);
@@ -1793,17 +1793,9 @@ void video_window(gbm3d_ctx* c, float* const* pads, int P, int m, int n, int F, 
   G.F = F;
   G.m = m;
   G.n = n;
-  G.U = U;
-  G.W = W;
+  G.Y = Y;
+  G.nn = nn;
   launched(c, launch_aggregate_video(G, c->st), "aggregate_video");
-}
-
-__global__ void k_video_accum(const double* __restrict__ U, const double* __restrict__ W, size_t n,
-                              float* __restrict__ Y, float* __restrict__ nn) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    Y[i] = (float)((double)Y[i] + U[i]);  // the reference's Y and nn are single arrays
-    nn[i] = (float)((double)nn[i] + W[i]);
-  }
 }
 
 // out frame (k - hw) += (Y ./ nn)(r + s, c + s) of frame k (the shift back), cropped to m0 x n0
@@ -1853,8 +1845,6 @@ void pipeline_video(gbm3d_ctx* c, const double* I, int m0, int n0, int Kf, doubl
   }
   float* Y = buf<float>(c, "v.Y", px * Kf);
   float* nn = buf<float>(c, "v.nn", px * Kf);
-  double* U = buf<double>(c, "v.U", px * F);
-  double* W = buf<double>(c, "v.W", px * F);
   double* acc = buf<double>(c, "v.acc", px0 * nOut);
   uint32_t* S = buf<uint32_t>(c, "v.S", (size_t)K * (Mp / d) * (Np / d));
   float* vol = buf<float>(c, "v.vol", px * K);
@@ -1864,12 +1854,16 @@ void pipeline_video(gbm3d_ctx* c, const double* I, int m0, int n0, int Kf, doubl
     const int s = o->matchSpins[ii];
     ck(c, cudaMemsetAsync(Y, 0, px * Kf * sizeof(float), c->st), "memset");
     ck(c, cudaMemsetAsync(nn, 0, px * Kf * sizeof(float), c->st), "memset");
+    // the search image of frame k (circshift(I3, [s, s, 0])) stays in buffer k mod F while windows hold it
+    auto pad_of = [&](int k) { return pads[k % F]; };
+    auto build_pad = [&](int k) { launched(c, launch_make_pad(fr + px * k, Mp, Np, d, s, pad_of(k), P, c->st), "make_pad"); };
+    for (int k = 0; k < F - 1; ++k) build_pad(k);
     for (int jj = hw; jj < Kf - hw; ++jj) {
-      for (int q = 0; q < F; ++q)  // circshift(I3, [s, s, 0]) and matchBlocksV's search images
-        launched(c, launch_make_pad(fr + px * (jj - hw + q), Mp, Np, d, s, pads[q], P, c->st), "make_pad");
-      video_window(c, pads.data(), P, Mp, Np, F, d, K, o->levels, o->cycleSpin, tau.data(), bk, S, vol, U, W);
-      k_video_accum<<<1184, 256, 0, c->st>>>(U, W, px * F, Y + px * (jj - hw), nn + px * (jj - hw));
-      launched(c, cudaGetLastError(), "video_accum");
+      build_pad(jj + hw);
+      std::vector<float*> wp(F);
+      for (int q = 0; q < F; ++q) wp[q] = pad_of(jj - hw + q);
+      video_window(c, wp.data(), P, Mp, Np, F, d, K, o->levels, o->cycleSpin, tau.data(), bk, S, vol,
+                   Y + px * (jj - hw), nn + px * (jj - hw));
     }
     k_video_out<<<1184, 256, 0, c->st>>>(Y, nn, Mp, Np, m0, n0, hw, nOut, s, acc, ii == 0);
     launched(c, cudaGetLastError(), "video_out");
@@ -1956,8 +1950,7 @@ int gbm3d_denoiseAndAggregateV(gbm3d_ctx* c, const float* Volume, const uint32_t
     uint32_t* dS = buf<uint32_t>(c, "io.S", (size_t)K * M * N);
     ck(c, cudaMemcpyAsync(dV, Volume, px * K * 4, cudaMemcpyHostToDevice, c->st), "H2D");
     ck(c, cudaMemcpyAsync(dS, S, (size_t)K * M * N * 4, cudaMemcpyHostToDevice, c->st), "H2D");
-    float* vsum = run_wavelet_ht(c, dV, m, n, K, o->levels, o->cycleSpin, tau, bk, 0);
-    launched(c, launch_clamp01(vsum, px * K, c->st), "clamp");
+    float* vsum = run_wavelet_ht(c, dV, m, n, K, o->levels, o->cycleSpin, tau, bk, 0, nullptr, 0, true);
     float* wgt = buf<float>(c, "v.wgt", (size_t)M * N);
     launched(c, launch_ht_weights(vsum, m, n, M, N, d, K, nullptr, wgt, c->st), "ht_weights");
     double* dU = buf<double>(c, "v.U", px * frames);

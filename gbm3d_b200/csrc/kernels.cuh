@@ -148,6 +148,7 @@ struct SynthOut {
   // cycles a power of two: multiplying by inv = 1 / cycles is the same division
   int pow2;
   float inv;
+  int clamp1;  // with last: clamp at 1 too (denoiseAndAggregateV.m's Vavg)
 };
 // cols: the output columns (values computed for p, before the shift) to produce.
 cudaError_t launch_wav_synthesis(const float* bands, const float* approx, int Oy, int Ox, int Oz,
@@ -246,9 +247,11 @@ struct VideoAggArgs {
   int M, N, d, K, F, m, n;
   double* U;              // m x n x F
   double* W;
+  // instead of U and W: the sums are added to these (m x n x F, single), or null
+  float* Y;
+  float* nn;
 };
 cudaError_t launch_aggregate_video(const VideoAggArgs& A, cudaStream_t st);
-cudaError_t launch_clamp01(float* v, size_t n, cudaStream_t st);
 
 // ---- learned pilot (pilot.cu) ----------------------------------------------------------
 constexpr int PILOT_LAYERS = 8;

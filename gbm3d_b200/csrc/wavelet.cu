@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(256) k_wav_synthesis(const float* __restrict__
     if (o.last) {
       v = v / o.cycles;
       v = v > 0.f ? v : 0.f;
+      if (o.clamp1) v = fminf(v, 1.f);
     }
     *dst = v;
   }
@@ -554,6 +555,7 @@ __global__ void __launch_bounds__(32 * MW, 4) k_wav_synthesis_march(const float*
             if (o.last) {
               v = o.pow2 ? make_float2(v.x * o.inv, v.y * o.inv) : divide2(v, o.cycles);
               v = make_float2(v.x > 0.f ? v.x : 0.f, v.y > 0.f ? v.y : 0.f);
+              if (o.clamp1) v = make_float2(fminf(v.x, 1.f), fminf(v.y, 1.f));
             }
             float* p = dz[z] + cols[c];
             if (PAIR) {

@@ -91,7 +91,7 @@ def video(a):
                                                 C.byref(co), C.c_void_p(dY.data_ptr())))
     st = ctx.stage_times()
     fam = {k: ctx.kernel_time(k) for k in ("match_video", "wav_analysis", "wav_synthesis", "ht_weights",
-                                           "aggregate_video", "clamp", "make_pad", "video_accum", "video_out",
+                                           "aggregate_video", "make_pad", "video_out",
                                            "prep")}
     ctx.enable_timing(False)
     ctx.check(_lib.lib().gbm3d_ctx_synchronize(ctx.h))
