@@ -294,9 +294,29 @@ __global__ void __launch_bounds__(128) k_wiener(WienerArgs A) {
 // halves exchanged, which puts the 16-byte column reads of a page on distinct
 // banks; the page pitch of 72 does the same for the rows of four pages.  36 KB and 80
 // registers: six CTAs per SM (five 1.35 ms, four 1.50 ms at 4096^2).
-//   4096^2 at stride 7 1.60 -> 1.28 ms, 1024^2 dense 1.06 -> 0.86 ms (two spins); now at 84 % of
-// the shared-memory pipe (326 of 843 wavefronts per group are the gather: four
-// lines per 4-byte asynchronous copy) and 81 % of the issue slots (3.5 k instructions).
+//   4096^2 at stride 7 1.60 -> 1.28 ms, and 1.22 with packed sums (mat8: 3.5 -> 2.75 k
+// instructions per group); 1024^2 dense 1.06 -> 0.80 ms (two spins).  Now at 87 % of the
+// shared-memory pipe; 326 of 840 wavefronts per group are the gather, four
+// lines per 4-byte asynchronous copy (through registers: the same).
+// out[q] = sum_j M(q, j) v[j] (M column-major 8 x 8, a constant operand), each a serial
+// fmaf chain from 0 in ascending j, two rows per packed instruction
+__device__ __forceinline__ void mat8(const float* M, const float (&v)[8], float (&out)[8]) {
+  unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    unsigned long long vv;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(vv) : "f"(v[j]));
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      unsigned long long m;
+      asm("mov.b64 %0, {%1, %2};" : "=l"(m) : "f"(M[2 * q + 8 * j]), "f"(M[2 * q + 1 + 8 * j]));
+      asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[q]) : "l"(m), "l"(vv));
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) asm("mov.b64 {%0, %1}, %2;" : "=f"(out[2 * q]), "=f"(out[2 * q + 1]) : "l"(acc[q]));
+}
+
 template <int K>
 struct Wie8 {
   static constexpr int PG = 72, BUF = K * PG;
@@ -364,13 +384,7 @@ __global__ void __launch_bounds__(128, 6) k_wiener_8(WienerArgs A) {
       const float4 hi = *reinterpret_cast<const float4*>(x + D * r + (h0 ^ 4));
       const float c[D] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
       float P[D];
-#pragma unroll
-      for (int q = 0; q < D; ++q) {
-        float acc = 0.f;
-#pragma unroll
-        for (int jj = 0; jj < D; ++jj) acc = fmaf(A.T[q + jj * D], c[jj], acc);
-        P[q] = acc;
-      }
+      mat8(A.T, c, P);
       *reinterpret_cast<float4*>(x + D * r + h0) = make_float4(P[0], P[1], P[2], P[3]);
       *reinterpret_cast<float4*>(x + D * r + (h0 ^ 4)) = make_float4(P[4], P[5], P[6], P[7]);
     }
@@ -379,13 +393,10 @@ __global__ void __launch_bounds__(128, 6) k_wiener_8(WienerArgs A) {
       float P[D];
 #pragma unroll
       for (int n = 0; n < D; ++n) P[n] = x[D * n + (r ^ (n & 4))];
+      float Y[D];
+      mat8(A.T, P, Y);
 #pragma unroll
-      for (int l = 0; l < D; ++l) {
-        float acc = 0.f;
-#pragma unroll
-        for (int n = 0; n < D; ++n) acc = fmaf(P[n], A.T[l + n * D], acc);
-        x[D * l + (r ^ (l & 4))] = acc;
-      }
+      for (int l = 0; l < D; ++l) x[D * l + (r ^ (l & 4))] = Y[l];
     }
   }
   __syncwarp();
@@ -454,26 +465,21 @@ __global__ void __launch_bounds__(128, 6) k_wiener_8(WienerArgs A) {
       float Y[D];
 #pragma unroll
       for (int n = 0; n < D; ++n) Y[n] = y[D * n + (r ^ (n & 4))];
+      float P[D];
+      mat8(A.Ti, Y, P);
 #pragma unroll
-      for (int l = 0; l < D; ++l) {
-        float acc = 0.f;
-#pragma unroll
-        for (int n = 0; n < D; ++n) acc = fmaf(Y[n], A.Ti[l + n * D], acc);
-        y[D * l + (r ^ (l & 4))] = acc;
-      }
+      for (int l = 0; l < D; ++l) y[D * l + (r ^ (l & 4))] = P[l];
     }
     __syncwarp();
     {
       const float4 lo = *reinterpret_cast<const float4*>(y + D * r + h0);
       const float4 hi = *reinterpret_cast<const float4*>(y + D * r + (h0 ^ 4));
       const float c[D] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-      float z[D];
+      float X[D], z[D];
+      mat8(A.Ti, c, X);
 #pragma unroll
       for (int q = 0; q < D; ++q) {
-        float acc = 0.f;
-#pragma unroll
-        for (int jj = 0; jj < D; ++jj) acc = fmaf(A.Ti[q + jj * D], c[jj], acc);
-        float v = acc > 0.f ? acc : 0.f;
+        float v = X[q] > 0.f ? X[q] : 0.f;
         if (A.clamp_one && v > 1.f) v = 1.f;
         z[q] = wc[q] * v;  // weight.*blocks(:,:,i) (:84-90)
       }
