@@ -360,22 +360,46 @@ __global__ void k_shift_copy(const float* __restrict__ v, int Mp, int Np, int s,
   out[r + (size_t)c * Mp] = v[pmod(r + s, Mp) + (size_t)pmod(c + s, Np) * Mp];
 }
 
-__global__ void k_add_f(const float* __restrict__ v, double* __restrict__ acc, size_t n) {
-  size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) acc[i] = acc[i] + (double)v[i];
-}
-
-// out = a ./ b on the padded grid (double), its single copy, and the m x n crop.
-__global__ void k_ratio(const double* __restrict__ a, const double* __restrict__ b, int Mp, int Np,
-                        double* __restrict__ full, float* __restrict__ full_f, double* __restrict__ crop,
-                        int m, int n) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
-  if (r >= Mp || c >= Np) return;
-  const size_t o = r + (size_t)c * Mp;
-  const double v = a[o] / b[o];
-  if (full) full[o] = v;
-  if (full_f) full_f[o] = (float)v;
-  if (crop && r < m && c < n) crop[r + (size_t)c * m] = v;
+// The last spin's accumulation and the ratio of the sums in one pass: v = (ua + u) ./
+// (wa + w + stale weights), u and w shifted back by the spin, everything in
+// double (ua, wa null for a single spin).  v goes to the padded single image
+// and, cropped to m x n, to up to two outputs.  With the sums written out and
+// read again this took 157 + 165 us for both steps at 4096^2, now 191 in all
+// (bound by the divisions and the latency in front of them; one column per
+// thread: 256).
+constexpr int FCOLS = 4;  // columns per thread: their loads and divisions overlap
+__global__ void __launch_bounds__(256) k_finish(const float* __restrict__ u, const float* __restrict__ w, int Mp, int Np,
+                                                int s, const double* __restrict__ ua, const double* __restrict__ wa,
+                                                const float* __restrict__ stale, int nstale,
+                                                float* __restrict__ full_f, double* __restrict__ crop,
+                                                double* __restrict__ crop2, int m, int n) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x, c0 = blockIdx.y * FCOLS;
+  if (r >= Mp) return;
+  const int sr = shift_index(r, s, Mp);
+  double x[FCOLS], y[FCOLS];
+#pragma unroll
+  for (int q = 0; q < FCOLS; ++q) {
+    const int c = min(c0 + q, Np - 1);
+    const size_t src = sr + (size_t)shift_index(c, s, Np) * Mp, o = r + (size_t)c * Mp;
+    x[q] = (double)__ldg(u + src);
+    y[q] = (double)__ldg(w + src);
+    if (ua) {
+      x[q] = __ldg(ua + o) + x[q];
+      y[q] = __ldg(wa + o) + y[q];
+    }
+    for (int t = 0; t < nstale; ++t) y[q] = y[q] + (double)__ldg(stale + o + (size_t)t * Mp * Np);
+  }
+#pragma unroll
+  for (int q = 0; q < FCOLS; ++q) {
+    const int c = c0 + q;
+    if (c >= Np) break;
+    const double v = x[q] / y[q];
+    if (full_f) full_f[r + (size_t)c * Mp] = (float)v;
+    if (r < m && c < n) {
+      if (crop) crop[r + (size_t)c * m] = v;
+      if (crop2) crop2[r + (size_t)c * m] = v;
+    }
+  }
 }
 
 dim3 grid2(int rows, int cols) { return dim3((rows + 255) / 256, cols); }
@@ -995,9 +1019,9 @@ void pipeline(gbm3d_ctx* c, const double* dI, int m, int n, double sigma, const 
 
   float* Us = buf<float>(c, "p.Us", px);
   float* Ws = buf<float>(c, "p.Ws", px);
-  double* Ua = buf<double>(c, "p.Ua", px);
-  double* Wa = buf<double>(c, "p.Wa", px);
-  double* U1d = buf<double>(c, "p.U1d", px);
+  const bool sums = nS > 1 || nW > 1;  // a single spin's sums never leave k_finish
+  double* Ua = sums ? buf<double>(c, "p.Ua", px) : nullptr;
+  double* Wa = sums ? buf<double>(c, "p.Wa", px) : nullptr;
   float* U1f = buf<float>(c, "p.U1f", px);
   const bool stale = o->form != 2 && o->Wiener && o->staleWeights && nW < nS;
   float* Wstale = stale ? buf<float>(c, "p.Wstale", px * (nS - nW)) : nullptr;
@@ -1037,20 +1061,20 @@ void pipeline(gbm3d_ctx* c, const double* dI, int m, int n, double sigma, const 
     }
     run_ht(c, vol, S1, cnt1, M1, N1, d, d2, K, o->levels, o->cycleSpin, tau.data(), bk, Us, Ws, o->filtType, st1,
            strip ? &plan.s1[ii] : nullptr);
-    k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua, Wa, ii == 0);
-    launched(c, cudaGetLastError(), "accum");
+    if (ii + 1 < nS) {
+      k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua, Wa, ii == 0);
+      launched(c, cudaGetLastError(), "accum");
+    } else {
+      k_finish<<<grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, ii ? Ua : nullptr, ii ? Wa : nullptr, nullptr, 0, U1f,
+                                                 dU1, o->Wiener ? nullptr : dU, m, n);
+      launched(c, cudaGetLastError(), "ratio");
+    }
     if (stale && ii >= nW) {
       k_shift_copy<<<grid2(Mp, Np), 256, 0, c->st>>>(Ws, Mp, Np, s, Wstale + (size_t)(ii - nW) * px);
       launched(c, cudaGetLastError(), "shift_copy");
     }
   }
-  k_ratio<<<grid2(Mp, Np), 256, 0, c->st>>>(Ua, Wa, Mp, Np, U1d, U1f, dU1, m, n);
-  launched(c, cudaGetLastError(), "ratio");
-  if (!o->Wiener) {
-    k_ratio<<<grid2(Mp, Np), 256, 0, c->st>>>(Ua, Wa, Mp, Np, nullptr, nullptr, dU, m, n);
-    launched(c, cudaGetLastError(), "ratio");
-    return;
-  }
+  if (!o->Wiener) return;
   }
 
   // step 2: empirical Wiener estimate over the Wiener match spins
@@ -1088,16 +1112,15 @@ void pipeline(gbm3d_ctx* c, const double* dI, int m, int n, double sigma, const 
       launched(c, cudaGetLastError(), "window_counts");
     }
     run_wiener_agg(c, A, dw, d2, Us, Ws, strip ? plan.s2[ii].agg : ColRange(), cnt2);
-    k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua, Wa, ii == 0);
-    launched(c, cudaGetLastError(), "accum");
-  }
-  if (stale)
-    for (int ii = nW; ii < nS; ++ii) {
-      k_add_f<<<(unsigned)((px + 255) / 256), 256, 0, c->st>>>(Wstale + (size_t)(ii - nW) * px, Wa, px);
-      launched(c, cudaGetLastError(), "add");
+    if (ii + 1 < nW) {
+      k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua, Wa, ii == 0);
+      launched(c, cudaGetLastError(), "accum");
+    } else {
+      k_finish<<<grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, ii ? Ua : nullptr, ii ? Wa : nullptr, Wstale,
+                                                 stale ? nS - nW : 0, nullptr, dU, nullptr, m, n);
+      launched(c, cudaGetLastError(), "ratio");
     }
-  k_ratio<<<grid2(Mp, Np), 256, 0, c->st>>>(Ua, Wa, Mp, Np, nullptr, nullptr, dU, m, n);
-  launched(c, cudaGetLastError(), "ratio");
+  }
 }
 
 }  // namespace
@@ -1692,13 +1715,15 @@ void pipeline_rgb(gbm3d_ctx* c, const double* const* dI, int m, int n, double si
       std::vector<double> tau(tau1);
       for (auto& t : tau) t *= csig[ch];
       run_ht(c, vol, S1, cnt1, M1, N1, d, d2, K, o->levels, o->cycleSpin, tau.data(), bk, Us, Ws, o->filtType, st1);
-      k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua[ch], Wa[ch], ii == 0);
-      launched(c, cudaGetLastError(), "accum");
+      if (ii + 1 < nS) {
+        k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua[ch], Wa[ch], ii == 0);
+        launched(c, cudaGetLastError(), "accum");
+      } else {
+        k_finish<<<grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, ii ? Ua[ch] : nullptr, ii ? Wa[ch] : nullptr,
+                                                   nullptr, 0, U1f[ch], nullptr, nullptr, m, n);
+        launched(c, cudaGetLastError(), "ratio");
+      }
     }
-  }
-  for (int ch = 0; ch < 3; ++ch) {
-    k_ratio<<<grid2(Mp, Np), 256, 0, c->st>>>(Ua[ch], Wa[ch], Mp, Np, nullptr, U1f[ch], nullptr, m, n);
-    launched(c, cudaGetLastError(), "ratio");
   }
 
   // step 2: matching on the luma pilot, per-channel Wiener filtering
@@ -1726,13 +1751,15 @@ void pipeline_rgb(gbm3d_ctx* c, const double* const* dI, int m, int n, double si
       A.s = st2;
       fill_wiener_consts(A, dw, &csig[ch], 0, 0);
       run_wiener_agg(c, A, dw, d2, Us, Ws);
-      k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua[ch], Wa[ch], ii == 0);
-      launched(c, cudaGetLastError(), "accum");
+      if (ii + 1 < nW) {
+        k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua[ch], Wa[ch], ii == 0);
+        launched(c, cudaGetLastError(), "accum");
+      } else {
+        k_finish<<<grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, ii ? Ua[ch] : nullptr, ii ? Wa[ch] : nullptr,
+                                                   nullptr, 0, nullptr, opp[ch], nullptr, m, n);
+        launched(c, cudaGetLastError(), "ratio");
+      }
     }
-  }
-  for (int ch = 0; ch < 3; ++ch) {
-    k_ratio<<<grid2(Mp, Np), 256, 0, c->st>>>(Ua[ch], Wa[ch], Mp, Np, nullptr, nullptr, opp[ch], m, n);
-    launched(c, cudaGetLastError(), "ratio");
   }
   k_opp<<<592, 256, 0, c->st>>>(opp[0], opp[1], opp[2], pm, dU[0], dU[1], dU[2], 1);
   launched(c, cudaGetLastError(), "opp");
