@@ -146,6 +146,50 @@ __global__ void __launch_bounds__(128, 7) k_match(const __grid_constant__ CUtens
   match_ref<D, D2>(A, &tmap, g, win, lst, mbar, phase, lane);
 }
 
+// Few references of a large patch: a CTA per reference, each warp the distances of
+// D2 / 4 candidate columns, warp 0 the selection and the gathers.  One warp per
+// reference takes 24 us however few there are at patch 16 (16.4 k instructions of
+// exact SSD in a row); split it takes 15 for the 48 of 128 x 96.
+template <int D, int D2>
+__global__ void __launch_bounds__(128) k_match_split(const __grid_constant__ CUtensorMap tmap, MatchArgs A) {
+  constexpr int WD = D + D2 - 1, WP = win_pitch(WD), NB = D2 / 4;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  float* win = reinterpret_cast<float*>(smem_raw);
+  float* keys = win + win_floats(WD);                                       // [b][lane]
+  uint32_t* lst = reinterpret_cast<uint32_t*>(keys + D2 * 32);
+  __shared__ uint64_t mbar;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = window_group(blockIdx.x, A.g0, A.gn, A.M * A.N);
+  if (g < 0) return;  // the same for the whole CTA
+  const int i = g % A.M, j = g / A.M, y0 = i * A.s, o = y0 & 3;
+  if (threadIdx.x == 0) {
+    tc::mbar_init(&mbar, 1);
+    tc::fence_mbar_init();
+    tc::mbar_expect_tx(&mbar, WP * WD * (int)sizeof(float));
+    tc::tma_load_2d(win, &tmap, y0 - o, j * A.s, &mbar);
+  }
+  __syncthreads();  // the barrier word is initialised
+  const bool ok = tc::mbar_wait(&mbar, 0, MATCH_WAIT_CYCLES);
+  if (!__syncthreads_and(ok)) {
+    // give the copy the full limit again before the buffer goes away, report
+    if (!ok) tc::mbar_wait(&mbar, 0, MATCH_WAIT_CYCLES);
+    if (threadIdx.x == 0 && A.err) atomicOr(A.err, 4);
+    return;
+  }
+  const float* wv = win + o;
+  float part[NB];
+  exact_ssd<D, D2, NB>(wv, lane, warp * NB, part);
+#pragma unroll
+  for (int b = 0; b < NB; ++b) keys[(warp * NB + b) * 32 + lane] = part[b];
+  __syncthreads();
+  if (warp) return;
+  float acc[D2];
+#pragma unroll
+  for (int b = 0; b < D2; ++b) acc[b] = keys[b * 32 + lane];
+  const int count = select_group<D, D2>(A, wv, acc, lst, lane);
+  emit_group<D, D2>(A, g, i, j, wv, lst + 64, count, lane);
+}
+
 // List mode: the references A.list[0 .. *A.list_count), grid-stride over the list.
 template <int D, int D2>
 __global__ void __launch_bounds__(128) k_match_list(const __grid_constant__ CUtensorMap tmap, MatchArgs A) {
@@ -188,6 +232,19 @@ static cudaError_t launch_match_t(const MatchArgs& A, cudaStream_t st) {
 }
 
 template <int D, int D2>
+static cudaError_t launch_match_split(const MatchArgs& A, cudaStream_t st) {
+  constexpr int WD = D + D2 - 1;
+  const size_t sm = (size_t)(win_floats(WD) + D2 * 32 + 224) * sizeof(float);
+  CUtensorMap tm;
+  if (!encode_search_map(&tm, A.pad, A.R, A.Q, A.P, win_pitch(WD), WD)) return cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute(k_match_split<D, D2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  if (A.gn < 0) return cudaSuccess;  // an empty window
+  k_match_split<D, D2><<<A.gn > 0 ? A.gn : A.M * A.N, 128, sm, st>>>(tm, A);
+  return cudaGetLastError();
+}
+
+template <int D, int D2>
 static cudaError_t launch_match_list_t(const MatchArgs& A, cudaStream_t st) {
   constexpr int WD = D + D2 - 1;
   const size_t sm = MatchSmem<D, D2>::BYTES;
@@ -218,6 +275,16 @@ bool match_supported(int d, int d2) {
 cudaError_t launch_match(int d, int d2, const MatchArgs& A, cudaStream_t st) {
   if (A.s < 1 || A.s > d) return cudaErrorInvalidValue;
   if (match_bound_supported(d, d2, A)) return launch_match_bound(A, st);
+  // patches 16 and 32, at most two references per SM: split.  Both spins of step 1 at patch
+  // 16, us unsplit / split: 48 references 75 / 58, 256 77 / 65, 1024 98 / 119, 2304 149 / 168
+  // (a split reference keeps three warps waiting for the selection); patch 32: 256 290 / 150,
+  // 1024 354 / 415.
+  const long groups = A.gn > 0 ? A.gn : (long)A.M * A.N;
+#define GBM3D_SPLIT_CASE(DD, DD2) \
+  if (d == DD && d2 == DD2 && groups <= 2 * 148) return launch_match_split<DD, DD2>(A, st);
+  GBM3D_SPLIT_CASE(16, 16) GBM3D_SPLIT_CASE(16, 24) GBM3D_SPLIT_CASE(16, 32)
+  GBM3D_SPLIT_CASE(32, 16) GBM3D_SPLIT_CASE(32, 24) GBM3D_SPLIT_CASE(32, 32)
+#undef GBM3D_SPLIT_CASE
 #define GBM3D_MATCH_CASE(DD, DD2) \
   if (d == DD && d2 == DD2) return A.gn ? launch_match_t<DD, DD2, true>(A, st) : launch_match_t<DD, DD2, false>(A, st);
   GBM3D_MATCH_CASE(8, 16) GBM3D_MATCH_CASE(8, 24) GBM3D_MATCH_CASE(8, 32)

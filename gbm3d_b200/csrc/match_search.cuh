@@ -15,34 +15,28 @@ __host__ __device__ constexpr int win_pitch(int wd) { return (wd + 3 + 3) & ~3; 
 __host__ __device__ constexpr int win_floats(int wd) { return (win_pitch(wd) * wd + 31) & ~31; }
 constexpr long long MATCH_WAIT_CYCLES = 4000000000LL;  // ~2 s at 2 GHz
 
-// The exhaustive search of one reference by one warp: wv is the reference's
-// window (row 0, column 0; column pitch win_pitch) in shared memory, lst 224
-// words (keys, indices, S and the bounded set).  Leaves the group's 1-based
-// window indices in lst[64 ..] and returns their count.
-template <int D, int D2>
-__device__ __forceinline__ int search_exhaustive(const MatchArgs& A, const float* wv, uint32_t* lst, const int lane) {
-  constexpr int WD = D + D2 - 1;  // window rows/cols that candidates touch
-  constexpr int WP = win_pitch(WD);
+// Exact SSD of the lane's candidates a = lane (a < D2), b = b0 .. b0 + NB - 1: wv is the
+// reference's window (row 0, column 0; column pitch win_pitch) in shared memory.
+// Candidate b sees t = x(r, c) - y, acc = fmaf(t, t, acc) in (r, c) order (c = xw - b
+// ascends with the window column xw).
+template <int D, int D2, int NB>
+__device__ __forceinline__ void exact_ssd(const float* wv, const int lane, const int b0, float (&acc)[NB]) {
+  constexpr int WP = win_pitch(D + D2 - 1);
   constexpr int H = D2 / 2;
-
-  // ---- exact SSD for the lane's candidates (a = lane, b = 0..D2-1) ----------
-  // Candidate b sees t = x(r, c) - y, acc = fmaf(t, t, acc) in (r, c) order
-  // (c = xw - b ascends with the window column xw).
-  float acc[D2];
 #pragma unroll
-  for (int b = 0; b < D2; ++b) acc[b] = 0.f;
+  for (int b = 0; b < NB; ++b) acc[b] = 0.f;
   const int a = lane < D2 ? lane : 0;
 #pragma unroll 1
   for (int r = 0; r < D; ++r) {
     float xr[D];
 #pragma unroll
     for (int c = 0; c < D; ++c) xr[c] = wv[(H + r) + (H + c) * WP];
-    const float* wrow = wv + (a + r);
+    const float* wrow = wv + (a + r) + b0 * WP;
 #pragma unroll
-    for (int xw = 0; xw < WD; ++xw) {
+    for (int xw = 0; xw < D + NB - 1; ++xw) {
       const float w = wrow[xw * WP];
 #pragma unroll
-      for (int b = 0; b < D2; ++b) {
+      for (int b = 0; b < NB; ++b) {
         const int c = xw - b;
         if (c >= 0 && c < D) {
           const float t = xr[c] - w;
@@ -51,7 +45,17 @@ __device__ __forceinline__ int search_exhaustive(const MatchArgs& A, const float
       }
     }
   }
+}
 
+// Selection of a reference's group by one warp from its exact distances: lane a
+// holds the candidates (a, b), b = 0 .. D2-1.  lst: 224 words (keys, indices, S and the bounded set).
+// Leaves the group's 1-based window indices in lst[64 ..] and returns their count.
+template <int D, int D2>
+__device__ __forceinline__ int select_group(const MatchArgs& A, const float* wv, const float (&acc)[D2], uint32_t* lst,
+                                            const int lane) {
+  constexpr int WP = win_pitch(D + D2 - 1);
+  constexpr int H = D2 / 2;
+  const int a = lane < D2 ? lane : 0;
   // ---- selection -------------------------------------------------------------
   const unsigned FULL = 0xffffffffu;
   uint32_t key[D2];
@@ -230,6 +234,14 @@ __device__ __forceinline__ int search_exhaustive(const MatchArgs& A, const float
   }
   __syncwarp();
   return count;
+}
+
+// The exhaustive search of one reference by one warp.
+template <int D, int D2>
+__device__ __forceinline__ int search_exhaustive(const MatchArgs& A, const float* wv, uint32_t* lst, const int lane) {
+  float acc[D2];
+  exact_ssd<D, D2, D2>(wv, lane, 0, acc);
+  return select_group<D, D2>(A, wv, acc, lst, lane);
 }
 
 // Write the group's S and count, and the optional gathers.
