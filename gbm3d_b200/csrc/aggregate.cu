@@ -50,6 +50,11 @@ constexpr int WB = 8;                              // walk batch: entries tested
 // sparse reference grids (fewer entries per tile) and lets more CTAs reside.
 template <int D, int D2, bool WIE, bool KAHAN, int CAPC>
 __global__ void __launch_bounds__(NTC) k_aggregate_cta(AggArgs A) {
+  const float* blocks = A.blocks;
+  const float* gw = A.gw;
+  const uint32_t* Sg = A.S;
+  const int32_t* counts = A.cnt;
+  begin_after_previous(blocks, gw, Sg, counts);
   extern __shared__ int smi[];
   __shared__ int wcnt[NTC / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
@@ -112,8 +117,8 @@ __global__ void __launch_bounds__(NTC) k_aggregate_cta(AggArgs A) {
       for (int t = 0; t < WB; ++t) {
         en[t] = lst[e0 + t];
         cov[t] = (en[t].x >> lane) & 1;
-        val[t] = cov[t] ? __ldg(A.blocks + ((size_t)(unsigned)(en[t].y + voff))) : 0.f;
-        if (WIE) wv[t] = cov[t] ? __ldg(A.gw + ((size_t)(unsigned)(en[t].z + woff))) : 0.f;
+        val[t] = cov[t] ? __ldg(blocks + ((size_t)(unsigned)(en[t].y + voff))) : 0.f;
+        if (WIE) wv[t] = cov[t] ? __ldg(gw + ((size_t)(unsigned)(en[t].z + woff))) : 0.f;
         else wv[t] = cov[t] ? win[woff - en[t].z] : 0.f;
       }
 #pragma unroll
@@ -195,9 +200,9 @@ __global__ void __launch_bounds__(NTC) k_aggregate_cta(AggArgs A) {
       // the count, the match index and the group weight are independent
       // loads: all three in flight before the count test (S holds K entries
       // per group whatever the count)
-      const int nm = A.cnt ? __ldg(A.cnt + g) : K;
-      const int eS = (int)__ldg(A.S + (size_t)g * K + k) - 1;
-      const float gwv = WIE ? 0.f : __ldg(A.gw + g);
+      const int nm = counts ? __ldg(counts + g) : K;
+      const int eS = (int)__ldg(Sg + (size_t)g * K + k) - 1;
+      const float gwv = WIE ? 0.f : __ldg(gw + g);
       if (k < nm) {
         const int e = eS;
         const int r0 = i * s + e % D2 - PR0, c0 = j * s + e / D2 - PC0;
@@ -254,7 +259,7 @@ static cudaError_t launch_px_cap(const AggArgs& A, cudaStream_t st) {
   tile_span(A.cols, A.n, CC, B.ct0, nt);
   if (nt == 0) return cudaSuccess;
   const int tiles = ((A.m + CR - 1) / CR) * nt;
-  k_aggregate_cta<D, D2, WIE, KAHAN, CAPC><<<tiles, NTC, sm, st>>>(B);
+  launch_next(k_aggregate_cta<D, D2, WIE, KAHAN, CAPC>, tiles, NTC, sm, st, B);
   return cudaGetLastError();
 }
 
@@ -301,6 +306,11 @@ struct AggBlk {
 
 template <int D, int D2, bool WIE, bool KAHAN, int RR, int RC>
 __global__ void __launch_bounds__(32) k_aggregate_blk(AggArgs A) {
+  const float* blocks = A.blocks;
+  const float* gw = A.gw;
+  const uint32_t* Sg = A.S;
+  const int32_t* counts = A.cnt;
+  begin_after_previous(blocks, gw, Sg, counts);
   using G = AggBlk<D, KAHAN, RR, RC>;
   constexpr int PT = G::PT, SV = G::SV, NB = G::NB, EB = G::EB;
   constexpr int NP = D * D / 32, CSTEP = 32 / D;  // pixels per lane, block columns between them
@@ -326,8 +336,8 @@ __global__ void __launch_bounds__(32) k_aggregate_blk(AggArgs A) {
 
   // this lane's block pixels: (pr, pc + CSTEP q)
   const int pr = lane % D, pc = lane / D;
-  const float* vsrc = A.blocks + lane;
-  const float* wsrc = WIE ? A.gw + lane : nullptr;
+  const float* vsrc = blocks + lane;
+  const float* wsrc = WIE ? gw + lane : nullptr;
   float* apx = acc + (pr + PT * pc) * SV;
   float mask[NP];
 #pragma unroll
@@ -424,9 +434,9 @@ __global__ void __launch_bounds__(32) k_aggregate_blk(AggArgs A) {
       int i, j, k;
       decode(min(base + 32 * u + lane, total - 1), i, j, k);
       const int g = i + A.M * j;
-      C.nm[u] = A.cnt ? __ldg(A.cnt + g) : K;
-      C.e[u] = (int)__ldg(A.S + (size_t)g * K + k) - 1;
-      C.gw[u] = WIE ? 0.f : __ldg(A.gw + g);
+      C.nm[u] = counts ? __ldg(counts + g) : K;
+      C.e[u] = (int)__ldg(Sg + (size_t)g * K + k) - 1;
+      C.gw[u] = WIE ? 0.f : __ldg(gw + g);
     }
   };
   __syncwarp();
@@ -451,7 +461,7 @@ __global__ void __launch_bounds__(32) k_aggregate_blk(AggArgs A) {
         en.z = WIE ? g * (D * D) : __float_as_int(cur.gw[u]);
         en.w = 0;
         lst[cnt + __popc(bal & below)] = en;
-        prefetch_l2<D * D>(A.blocks + (size_t)(unsigned)en.y);
+        prefetch_l2<D * D>(blocks + (size_t)(unsigned)en.y);
       }
       cnt += __popc(bal);
     }
@@ -482,7 +492,7 @@ static cudaError_t launch_blk(const AggArgs& A, cudaStream_t st) {
   int nt;
   tile_span(A.cols, A.n, RC, B.ct0, nt);
   if (nt == 0) return cudaSuccess;
-  k_aggregate_blk<D, D2, WIE, KAHAN, RR, RC><<<((A.m + RR - 1) / RR) * nt, 32, sm, st>>>(B);
+  launch_next(k_aggregate_blk<D, D2, WIE, KAHAN, RR, RC>, ((A.m + RR - 1) / RR) * nt, 32, sm, st, B);
   return cudaGetLastError();
 }
 

@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #define GBM3D_MAX_TAPS 16
 #define GBM3D_MAX_LEVELS 6
 
@@ -24,6 +26,43 @@ __host__ __device__ __forceinline__ int pmod(int a, int L) {
 // then circshift by h=d2/2).  Rows 0..h-1 hold image rows h..2h-1.
 __host__ __device__ __forceinline__ int pad_index(int r, int L, int h) {
   return r < h ? r + h : (r - h) % L;
+}
+
+// First statement of every kernel that launch_next() launches: wait until the
+// kernels before it on the stream are complete and their writes visible, then
+// let the next one's CTAs take the slots that this one leaves free.  The pointers
+// given are those read through __ldg or as const __restrict__ parameters: loads that
+// the compiler may take for constant over the kernel and move up.  They leave here with
+// a value of unknown origin, so that no such load can be made before the wait.
+template <class... P>
+__device__ __forceinline__ void begin_after_previous(P&... read_only) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (..., [](auto& p) { asm volatile("" : "+l"(p)::"memory"); }(read_only));
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launch with programmatic stream serialisation: the grid may be set up and its
+// CTAs made resident while the previous kernel's last ones still run, and each waits at
+// begin_after_previous().  Every kernel of a chain waits, so completion is transitive;
+// a plain launch, copy or event after it waits for the whole of it as ever.  Of
+// the 47 launches of a 128 x 96 call it saves 1.9 us each.
+template <class... P, class... Q>
+inline void launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Q&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  // in a captured graph plain edges: with several lanes the waiting CTAs hold slots
+  // that another lane's kernels could use (a batch of ten images: 16.8 against 16.2 ms)
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(st, &capture);
+  cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, std::forward<Q>(args)...);  // the caller reads cudaGetLastError()
 }
 
 // 4-byte asynchronous global -> shared copy: no register round trip, so all of

@@ -345,6 +345,7 @@ __global__ void k_or_flag(const int* __restrict__ flag, int* __restrict__ sticky
 
 __global__ void k_accum2(const float* __restrict__ u, const float* __restrict__ w, int Mp, int Np, int s,
                          double* __restrict__ ua, double* __restrict__ wa, int first) {
+  begin_after_previous(u, w);
   const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
   if (r >= Mp || c >= Np) return;
   const size_t src = shift_index(r, s, Mp) + (size_t)shift_index(c, s, Np) * Mp;
@@ -355,6 +356,7 @@ __global__ void k_accum2(const float* __restrict__ u, const float* __restrict__ 
 }
 
 __global__ void k_shift_copy(const float* __restrict__ v, int Mp, int Np, int s, float* __restrict__ out) {
+  begin_after_previous(v);
   const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
   if (r >= Mp || c >= Np) return;
   out[r + (size_t)c * Mp] = v[pmod(r + s, Mp) + (size_t)pmod(c + s, Np) * Mp];
@@ -373,6 +375,7 @@ __global__ void __launch_bounds__(256) k_finish(const float* __restrict__ u, con
                                                 const float* __restrict__ stale, int nstale,
                                                 float* __restrict__ full_f, double* __restrict__ crop,
                                                 double* __restrict__ crop2, int m, int n) {
+  begin_after_previous(u, w, ua, wa, stale);
   const int r = blockIdx.x * blockDim.x + threadIdx.x, c0 = blockIdx.y * FCOLS;
   if (r >= Mp) return;
   const int sr = shift_index(r, s, Mp);
@@ -1062,15 +1065,16 @@ void pipeline(gbm3d_ctx* c, const double* dI, int m, int n, double sigma, const 
     run_ht(c, vol, S1, cnt1, M1, N1, d, d2, K, o->levels, o->cycleSpin, tau.data(), bk, Us, Ws, o->filtType, st1,
            strip ? &plan.s1[ii] : nullptr);
     if (ii + 1 < nS) {
-      k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua, Wa, ii == 0);
+      launch_next(k_accum2, grid2(Mp, Np), 256, 0, c->st, Us, Ws, Mp, Np, s, Ua, Wa, ii == 0);
       launched(c, cudaGetLastError(), "accum");
     } else {
-      k_finish<<<grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, ii ? Ua : nullptr, ii ? Wa : nullptr, nullptr, 0, U1f,
-                                                 dU1, o->Wiener ? nullptr : dU, m, n);
+      launch_next(k_finish, grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st, Us, Ws, Mp, Np, s,
+                  ii ? Ua : nullptr, ii ? Wa : nullptr, nullptr, 0, U1f, dU1,
+                  o->Wiener ? nullptr : dU, m, n);
       launched(c, cudaGetLastError(), "ratio");
     }
     if (stale && ii >= nW) {
-      k_shift_copy<<<grid2(Mp, Np), 256, 0, c->st>>>(Ws, Mp, Np, s, Wstale + (size_t)(ii - nW) * px);
+      launch_next(k_shift_copy, grid2(Mp, Np), 256, 0, c->st, Ws, Mp, Np, s, Wstale + (size_t)(ii - nW) * px);
       launched(c, cudaGetLastError(), "shift_copy");
     }
   }
@@ -1113,11 +1117,12 @@ void pipeline(gbm3d_ctx* c, const double* dI, int m, int n, double sigma, const 
     }
     run_wiener_agg(c, A, dw, d2, Us, Ws, strip ? plan.s2[ii].agg : ColRange(), cnt2);
     if (ii + 1 < nW) {
-      k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua, Wa, ii == 0);
+      launch_next(k_accum2, grid2(Mp, Np), 256, 0, c->st, Us, Ws, Mp, Np, s, Ua, Wa, ii == 0);
       launched(c, cudaGetLastError(), "accum");
     } else {
-      k_finish<<<grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, ii ? Ua : nullptr, ii ? Wa : nullptr, Wstale,
-                                                 stale ? nS - nW : 0, nullptr, dU, nullptr, m, n);
+      launch_next(k_finish, grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st, Us, Ws, Mp, Np, s,
+                  ii ? Ua : nullptr, ii ? Wa : nullptr, Wstale,
+                  stale ? nS - nW : 0, nullptr, dU, nullptr, m, n);
       launched(c, cudaGetLastError(), "ratio");
     }
   }
@@ -1716,11 +1721,11 @@ void pipeline_rgb(gbm3d_ctx* c, const double* const* dI, int m, int n, double si
       for (auto& t : tau) t *= csig[ch];
       run_ht(c, vol, S1, cnt1, M1, N1, d, d2, K, o->levels, o->cycleSpin, tau.data(), bk, Us, Ws, o->filtType, st1);
       if (ii + 1 < nS) {
-        k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua[ch], Wa[ch], ii == 0);
+        launch_next(k_accum2, grid2(Mp, Np), 256, 0, c->st, Us, Ws, Mp, Np, s, Ua[ch], Wa[ch], ii == 0);
         launched(c, cudaGetLastError(), "accum");
       } else {
-        k_finish<<<grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, ii ? Ua[ch] : nullptr, ii ? Wa[ch] : nullptr,
-                                                   nullptr, 0, U1f[ch], nullptr, nullptr, m, n);
+        launch_next(k_finish, grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st, Us, Ws, Mp, Np, s,
+                    ii ? Ua[ch] : nullptr, ii ? Wa[ch] : nullptr, nullptr, 0, U1f[ch], nullptr, nullptr, m, n);
         launched(c, cudaGetLastError(), "ratio");
       }
     }
@@ -1752,11 +1757,11 @@ void pipeline_rgb(gbm3d_ctx* c, const double* const* dI, int m, int n, double si
       fill_wiener_consts(A, dw, &csig[ch], 0, 0);
       run_wiener_agg(c, A, dw, d2, Us, Ws);
       if (ii + 1 < nW) {
-        k_accum2<<<grid2(Mp, Np), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, Ua[ch], Wa[ch], ii == 0);
+        launch_next(k_accum2, grid2(Mp, Np), 256, 0, c->st, Us, Ws, Mp, Np, s, Ua[ch], Wa[ch], ii == 0);
         launched(c, cudaGetLastError(), "accum");
       } else {
-        k_finish<<<grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st>>>(Us, Ws, Mp, Np, s, ii ? Ua[ch] : nullptr, ii ? Wa[ch] : nullptr,
-                                                   nullptr, 0, nullptr, opp[ch], nullptr, m, n);
+        launch_next(k_finish, grid2(Mp, (Np + FCOLS - 1) / FCOLS), 256, 0, c->st, Us, Ws, Mp, Np, s,
+                    ii ? Ua[ch] : nullptr, ii ? Wa[ch] : nullptr, nullptr, 0, nullptr, opp[ch], nullptr, m, n);
         launched(c, cudaGetLastError(), "ratio");
       }
     }

@@ -62,6 +62,7 @@ bool encode_search_map(CUtensorMap* tm, const float* pad, int R, int Q, int P, i
 // multiple of 4; rows R .. P-1 of the pitch are never read as image rows).
 __global__ void k_make_pad(const float* __restrict__ img, int m, int n, int h, int spin,
                            float* __restrict__ pad, int P, int R, int Q) {
+  begin_after_previous(img);
   const int y0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int x = blockIdx.y;
   if (y0 >= P || x >= Q) return;
@@ -129,6 +130,7 @@ struct MatchSmem {
 // covers every group in order.
 template <int D, int D2, bool WIN>
 __global__ void __launch_bounds__(128, 7) k_match(const __grid_constant__ CUtensorMap tmap, MatchArgs A) {
+  begin_after_previous();
   using SM = MatchSmem<D, D2>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -152,6 +154,7 @@ __global__ void __launch_bounds__(128, 7) k_match(const __grid_constant__ CUtens
 // exact SSD in a row); split it takes 15 for the 48 of 128 x 96.
 template <int D, int D2>
 __global__ void __launch_bounds__(128) k_match_split(const __grid_constant__ CUtensorMap tmap, MatchArgs A) {
+  begin_after_previous();
   constexpr int WD = D + D2 - 1, WP = win_pitch(WD), NB = D2 / 4;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float* win = reinterpret_cast<float*>(smem_raw);
@@ -193,6 +196,7 @@ __global__ void __launch_bounds__(128) k_match_split(const __grid_constant__ CUt
 // List mode: the references A.list[0 .. *A.list_count), grid-stride over the list.
 template <int D, int D2>
 __global__ void __launch_bounds__(128) k_match_list(const __grid_constant__ CUtensorMap tmap, MatchArgs A) {
+  begin_after_previous();
   using SM = MatchSmem<D, D2>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -227,7 +231,7 @@ static cudaError_t launch_match_t(const MatchArgs& A, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   const int G = A.gn > 0 ? A.gn : A.M * A.N;
   if (A.gn < 0) return cudaSuccess;  // an empty window
-  k_match<D, D2, WIN><<<(G + 3) / 4, 128, sm, st>>>(tm, A);
+  launch_next(k_match<D, D2, WIN>, (G + 3) / 4, 128, sm, st, tm, A);
   return cudaGetLastError();
 }
 
@@ -240,7 +244,7 @@ static cudaError_t launch_match_split(const MatchArgs& A, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(k_match_split<D, D2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   if (A.gn < 0) return cudaSuccess;  // an empty window
-  k_match_split<D, D2><<<A.gn > 0 ? A.gn : A.M * A.N, 128, sm, st>>>(tm, A);
+  launch_next(k_match_split<D, D2>, A.gn > 0 ? A.gn : A.M * A.N, 128, sm, st, tm, A);
   return cudaGetLastError();
 }
 
@@ -255,7 +259,7 @@ static cudaError_t launch_match_list_t(const MatchArgs& A, cudaStream_t st) {
   const int G = A.M * A.N;
   // enough warps for the rare references a list holds; the rest exit at once
   const int blocks = std::min((G + 3) / 4, 2 * 148);
-  k_match_list<D, D2><<<blocks, 128, sm, st>>>(tm, A);
+  launch_next(k_match_list<D, D2>, blocks, 128, sm, st, tm, A);
   return cudaGetLastError();
 }
 
@@ -305,6 +309,7 @@ template <int D>
 __global__ void __launch_bounds__(256) k_gather_volume(const float* __restrict__ pad, int P, int M, int s, int d2,
                                                        int K, const uint32_t* __restrict__ S,
                                                        const int32_t* __restrict__ cnt, float* __restrict__ vol) {
+  begin_after_previous(pad, S, cnt);
   const int y = blockIdx.x * 256 + threadIdx.x, x = blockIdx.y, vm = M * D;
   if (y >= vm) return;
   const int i = y / D, r = y % D, j = x / D, c = x % D, h = d2 / 2;
@@ -328,9 +333,9 @@ cudaError_t launch_gather_volume(const float* pad, int P, int M, int N, int s, i
   const dim3 grid((M * d + 255) / 256, N * d);
   if (N * d > 65535) return cudaErrorInvalidValue;
   switch (d) {
-    case 8: k_gather_volume<8><<<grid, 256, 0, st>>>(pad, P, M, s, d2, K, S, cnt, vol); break;
-    case 16: k_gather_volume<16><<<grid, 256, 0, st>>>(pad, P, M, s, d2, K, S, cnt, vol); break;
-    case 32: k_gather_volume<32><<<grid, 256, 0, st>>>(pad, P, M, s, d2, K, S, cnt, vol); break;
+    case 8: launch_next(k_gather_volume<8>, grid, 256, 0, st, pad, P, M, s, d2, K, S, cnt, vol); break;
+    case 16: launch_next(k_gather_volume<16>, grid, 256, 0, st, pad, P, M, s, d2, K, S, cnt, vol); break;
+    case 32: launch_next(k_gather_volume<32>, grid, 256, 0, st, pad, P, M, s, d2, K, S, cnt, vol); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -341,7 +346,7 @@ cudaError_t launch_make_pad(const float* img, int m, int n, int d2, int spin, fl
   const int R = m + d2, Q = n + d2;
   dim3 grid((P / 4 + 255) / 256, Q);
   if ((P & 3) || P < R || (reinterpret_cast<uintptr_t>(pad) & 15)) return cudaErrorInvalidValue;
-  k_make_pad<<<grid, 256, 0, st>>>(img, m, n, d2 / 2, spin, pad, P, R, Q);
+  launch_next(k_make_pad, grid, 256, 0, st, img, m, n, d2 / 2, spin, pad, P, R, Q);
   return cudaGetLastError();
 }
 

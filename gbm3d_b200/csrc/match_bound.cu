@@ -59,6 +59,7 @@ constexpr int SCR = 96 + 2 * LCAND;
 // Groups of the column range [j0, j0 + nj): blockIdx.x = i + M (tile of four columns).
 __global__ void __launch_bounds__(128, 6) k_match_bound(const __grid_constant__ CUtensorMap tmap, MatchArgs A, int j0,
                                                         int nj, int nch) {
+  begin_after_previous();
   __shared__ __align__(128) float win[MAXCOL * WP];        // staged columns, pitch WP
   __shared__ __align__(16) float nrm[8 * MAXCH * WP];      // per position column: row sums, then -||w16||^2 / 2
   __shared__ __align__(16) __half w16[MAXCOL * HP];        // centred f16 window, pitch HP
@@ -331,7 +332,7 @@ cudaError_t launch_match_bound(const MatchArgs& A, cudaStream_t st) {
   const int from[2] = {lo, 0}, count[2] = {first, len - first};
   for (int q = 0; q < 2; ++q) {
     if (count[q] <= 0) continue;
-    k_match_bound<<<A.M * ((count[q] + NREF - 1) / NREF), 128, 0, st>>>(tm, A, from[q], count[q], nch);
+    launch_next(k_match_bound, A.M * ((count[q] + NREF - 1) / NREF), 128, 0, st, tm, A, from[q], count[q], nch);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }

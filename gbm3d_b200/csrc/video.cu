@@ -18,6 +18,7 @@ namespace {
 // minimum (the stable (value, index) order of mink).  S(1) is the reference.
 template <int D>
 __global__ void __launch_bounds__(128) k_match_video(VideoMatchArgs A) {
+  begin_after_previous();
   constexpr int WD = 2 * D, H = D / 2, DD = D * D;
   extern __shared__ unsigned long long keys[];   // F * D^2
   float* win = reinterpret_cast<float*>(keys + A.F * DD);  // WD x WD, column-major
@@ -144,6 +145,10 @@ constexpr int VT = 32, VTHREADS = 256, VLIST = 512;
 
 template <int D>
 __global__ void __launch_bounds__(VTHREADS) k_aggregate_video(VideoAggArgs A) {
+  const uint32_t* Sg = A.S;
+  const float* wgt = A.wgt;
+  const float* vsum = A.vsum;
+  begin_after_previous(Sg, wgt, vsum);
   constexpr int H = D / 2;
   __shared__ int4 lst[VLIST];
   __shared__ int wcnt[VTHREADS / 32];
@@ -162,7 +167,7 @@ __global__ void __launch_bounds__(VTHREADS) k_aggregate_video(VideoAggArgs A) {
       const int rr = lane - (short)(en.x & 0xffff), cc0 = warp - (en.x >> 16);
       const float wg = __int_as_float(en.z);
       const double dw = (double)wg;
-      const float* src = A.vsum + (((size_t)(unsigned)en.w << 32) | (unsigned)en.y) + rr;
+      const float* src = vsum + (((size_t)(unsigned)en.w << 32) | (unsigned)en.y) + rr;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int cc = cc0 + 8 * q;
@@ -180,7 +185,7 @@ __global__ void __launch_bounds__(VTHREADS) k_aggregate_video(VideoAggArgs A) {
     int4 en = make_int4(0, 0, 0, 0);
     if (t < total) {
       const int k = t % K, yx = t / K, y = ylo + yx / nx, x = xlo + yx % nx, g = y + A.M * x;
-      const int e = (int)__ldg(A.S + (size_t)g * K + k) - 1;
+      const int e = (int)__ldg(Sg + (size_t)g * K + k) - 1;
       const int a = e % D, b = (e / D) % D, f = e / (D * D);
       const int r = a + y * D - H, c = b + x * D - H;
       hit = f == fr && r >= 0 && c >= 0 && r < R0 + VT && r + D > R0 && c < C0 + VT && c + D > C0;
@@ -189,7 +194,7 @@ __global__ void __launch_bounds__(VTHREADS) k_aggregate_video(VideoAggArgs A) {
         const size_t o = (size_t)(y * D) + (size_t)A.m * (x * D) + mn * k;
         en.y = (int)(unsigned)o;
         en.w = (int)(o >> 32);
-        en.z = __float_as_int(__ldg(A.wgt + g));
+        en.z = __float_as_int(__ldg(wgt + g));
       }
     }
     const unsigned bal = __ballot_sync(0xffffffffu, hit);
@@ -250,7 +255,7 @@ cudaError_t launch_match_video(int d, const VideoMatchArgs& B, cudaStream_t st) 
   if (d == DD) {                                                                                            \
     cudaError_t e = cudaFuncSetAttribute(k_match_video<DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
     if (e != cudaSuccess) return e;                                                                         \
-    k_match_video<DD><<<G, 128, sm, st>>>(A);                                                               \
+    launch_next(k_match_video<DD>, G, 128, sm, st, A);                                                      \
     return cudaGetLastError();                                                                              \
   }
   GBM3D_VM_CASE(8) GBM3D_VM_CASE(16) GBM3D_VM_CASE(32)
@@ -261,9 +266,9 @@ cudaError_t launch_match_video(int d, const VideoMatchArgs& B, cudaStream_t st) 
 cudaError_t launch_aggregate_video(const VideoAggArgs& A, cudaStream_t st) {
   const dim3 grid((A.m + VT - 1) / VT, (A.n + VT - 1) / VT, A.F);
   switch (A.d) {
-    case 8: k_aggregate_video<8><<<grid, VTHREADS, 0, st>>>(A); break;
-    case 16: k_aggregate_video<16><<<grid, VTHREADS, 0, st>>>(A); break;
-    case 32: k_aggregate_video<32><<<grid, VTHREADS, 0, st>>>(A); break;
+    case 8: launch_next(k_aggregate_video<8>, grid, VTHREADS, 0, st, A); break;
+    case 16: launch_next(k_aggregate_video<16>, grid, VTHREADS, 0, st, A); break;
+    case 32: launch_next(k_aggregate_video<32>, grid, VTHREADS, 0, st, A); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

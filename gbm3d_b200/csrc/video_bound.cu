@@ -48,6 +48,7 @@ __device__ __forceinline__ float block_sum(float v, float* red, int warp, int la
 
 template <int F, int OCC>
 __global__ void __launch_bounds__(128, OCC) k_match_video_bound(VideoMatchArgs A) {
+  begin_after_previous();
   extern __shared__ __align__(16) unsigned char vsm[];
   float* win = reinterpret_cast<float*>(vsm);               // [column][row]
   __half* w16 = reinterpret_cast<__half*>(vsm + OFF_W16);   // centred f16 window, [column][row]
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(128, OCC) k_match_video_bound(VideoMatchArgs A
     const uint32_t s = sel[k];
     const int a = (int)(s % D), b = (int)((s / D) % D), f = (int)(s / DD);
     A.volume[(size_t)(i * D + r) + (size_t)A.m * (j * D + c) + mn * k] =
-        __ldg(A.pads[f] + (size_t)(i * D + a + r) + (size_t)(j * D + b + c) * A.P);
+        A.pads[f][(size_t)(i * D + a + r) + (size_t)(j * D + b + c) * A.P];
   }
 }
 
@@ -281,7 +282,7 @@ template <int F, int OCC>
 cudaError_t launch_vb(const VideoMatchArgs& A, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(k_match_video_bound<F, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VB_BYTES);
   if (e != cudaSuccess) return e;
-  k_match_video_bound<F, OCC><<<A.M * A.N, 128, VB_BYTES, st>>>(A);
+  launch_next(k_match_video_bound<F, OCC>, A.M * A.N, 128, VB_BYTES, st, A);
   return cudaGetLastError();
 }
 

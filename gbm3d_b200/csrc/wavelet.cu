@@ -288,6 +288,7 @@ __global__ void __launch_bounds__(32 * MW, 4) k_wav_analysis_march(const float* 
                                                                    int Lz, int shift, float* __restrict__ out,
                                                                    FastBank fb, LevelBands th, int ty, int x_lo,
                                                                    int x_len, int seg) {
+  begin_after_previous(in);
   constexpr int W = imax(LL, H0 + HN), HX = W / 2 - 1, HL = EVEN ? W / 2 : W / 2 - 1;
   constexpr int U = W > 2 ? W / 2 : 4, PD = 3;
   static_assert(W % 2 == 0 && (2 * U) % W == 0 && PD < U, "the window repeats every U steps");
@@ -416,6 +417,7 @@ __global__ void __launch_bounds__(32 * MW, 4) k_wav_synthesis_march(const float*
                                                                  const float* __restrict__ approx, int Oy, int Ox,
                                                                  int Oz, SynthOut o, FastBank fb, int ty, int x_lo,
                                                                  int x_len, int seg) {
+  begin_after_previous(bands, approx);
   constexpr int W = imax(S0 + SN, SH), HS = W / 2, RW = HS + 1, NST = 4, PQ = 40;
   static_assert(W % 2 == 0 && 32 + HS <= PQ && 8 * HS <= 64, "ring");
   __shared__ float ring[MW][NST][8][PQ];
@@ -633,7 +635,7 @@ static cudaError_t launch_analysis_march(const float* in, int Ly, int Lx, int Lz
   const int ty = (Ly / 2 + nout - 1) / nout, seg = march_segment(len, (long)ty * (Lz / 2));
   const dim3 grid((ty + MW - 1) / MW, (len + seg - 1) / seg, Lz / 2);
   auto kern = even ? k_wav_analysis_march<LL, H0, HN, true> : k_wav_analysis_march<LL, H0, HN, false>;
-  kern<<<grid, 32 * MW, 0, st>>>(in, Ly, Lx, Lz, shift, out, fb, th, ty, lo, len, seg);
+  launch_next(kern, grid, 32 * MW, 0, st, in, Ly, Lx, Lz, shift, out, fb, th, ty, lo, len, seg);
   return cudaGetLastError();
 }
 
@@ -645,7 +647,7 @@ static cudaError_t launch_synthesis_march(const float* bands, const float* appro
   const bool pair = (o.shift & 1) == 0;
   auto kern = o.first ? (pair ? k_wav_synthesis_march<S0, SN, SH, false, true> : k_wav_synthesis_march<S0, SN, SH, false, false>)
                       : (pair ? k_wav_synthesis_march<S0, SN, SH, true, true> : k_wav_synthesis_march<S0, SN, SH, true, false>);
-  kern<<<grid, 32 * MW, 0, st>>>(bands, approx, Oy, Ox, Oz, o, fb, ty, lo, len, seg);
+  launch_next(kern, grid, 32 * MW, 0, st, bands, approx, Oy, Ox, Oz, o, fb, ty, lo, len, seg);
   return cudaGetLastError();
 }
 
@@ -662,6 +664,7 @@ template <int D, bool GM>
 __global__ void __launch_bounds__(96) k_ht_weights_cta(const float* __restrict__ V, int m, int n, int M, int N, int K,
                                                        const int32_t* __restrict__ cnt, float* __restrict__ wgt,
                                                        int g0, int gn) {
+  begin_after_previous(V, cnt);
   constexpr int DM = D - 3, SL = D * D;
   extern __shared__ __align__(16) float sg[];
   __shared__ float sum[3];
@@ -829,6 +832,7 @@ template <bool GM>
 __global__ void __launch_bounds__(128) k_ht_weights_8(const float* __restrict__ V, int m, int n, int M, int N,
                                                       int K, const int32_t* __restrict__ cnt,
                                                       float* __restrict__ wgt, int g0, int gn) {
+  begin_after_previous(V, cnt);
   constexpr int D = 8, DM = D - 3, SL = D * D, SX = D * DM;
   extern __shared__ float shw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -903,13 +907,13 @@ cudaError_t launch_ht_weights(const float* Vavg, int m, int n, int M, int N, int
     auto kern = group_major ? k_ht_weights_8<true> : k_ht_weights_8<false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
     if (e != cudaSuccess) return e;
-    kern<<<(G + 3) / 4, 128, smb, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
+    launch_next(kern, (G + 3) / 4, 128, smb, st, Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
   } else if (d == 16 || (d == 32 && !group_major)) {
     auto kern = d == 32 ? k_ht_weights_cta<32, false> : group_major ? k_ht_weights_cta<16, true> : k_ht_weights_cta<16, false>;
     const size_t smb = (size_t)K * d * d * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
     if (e != cudaSuccess) return e;
-    kern<<<G, 96, smb, st>>>(Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
+    launch_next(kern, G, 96, smb, st, Vavg, m, n, M, N, K, cnt, wgt, g0, gn);
   } else if (group_major) {
     return cudaErrorInvalidValue;
   } else {

@@ -76,6 +76,7 @@ __device__ __forceinline__ void haar_rec(float* v, float cc) {
 
 template <int D, int K>
 __global__ void __launch_bounds__(128) k_wiener(WienerArgs A) {
+  begin_after_previous();
   constexpr int DD = D * D, GS = DD * K;
   // shared layout of one group: element (r, c) of slot page k at k*PG + r + D*c
   // (column-major pages).  The page stride D*D + D puts the 32/D pages a warp
@@ -325,6 +326,7 @@ struct Wie8 {
 
 template <int K>
 __global__ void __launch_bounds__(128, 6) k_wiener_8(WienerArgs A) {
+  begin_after_previous();
   constexpr int D = 8, DD = 64, PG = Wie8<K>::PG, BUF = Wie8<K>::BUF, GS = DD * K;
   extern __shared__ __align__(16) float smw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -497,7 +499,7 @@ static cudaError_t launch_wiener_8(const WienerArgs& A, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   const int G = A.gn > 0 ? A.gn : A.M * A.N;
   if (A.gn < 0) return cudaSuccess;  // an empty window
-  k_wiener_8<K><<<(G + 3) / 4, 128, sm, st>>>(A);
+  launch_next(k_wiener_8<K>, (G + 3) / 4, 128, sm, st, A);
   return cudaGetLastError();
 }
 
@@ -510,7 +512,7 @@ static cudaError_t launch_wiener_t(const WienerArgs& A, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   const int G = A.gn > 0 ? A.gn : A.M * A.N;
   if (A.gn < 0) return cudaSuccess;  // an empty window
-  k_wiener<D, K><<<(G + 3) / 4, 128, sm, st>>>(A);
+  launch_next(k_wiener<D, K>, (G + 3) / 4, 128, sm, st, A);
   return cudaGetLastError();
 }
 

@@ -1,0 +1,23 @@
+"""Launches that overlap the previous kernel's end (csrc/common.cuh, launch_next)
+against the plain launches of a captured graph: the same bits on repeated calls
+with changing inputs, from a single partial wave of CTAs to several."""
+import numpy as np
+import pytest
+
+from gbm3d_b200 import options, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,s", [(24, 24, 8), (65, 47, 3), (128, 96, 8), (301, 203, 3), (640, 480, 3)])
+def test_overlapped_launches_equal_captured(gpu, m, n, s):
+    import torch
+    from gbm3d_b200 import api
+    o = options.resolve_opts({"profile": "default"})
+    o.update(blockSize=8, blockSizeWie=8, matchSize=24, refStride=s, refStrideWie=s)
+    imgs = [torch.from_numpy(np.ascontiguousarray(synth.noisy_image(m, n, 25.0, seed=k)[1].T)).cuda() for k in (1, 2)]
+    captured = [x.clone() for x in api.GBM3D_batch(imgs, [25.0] * 2, o, use_graph=True)]
+    for _ in range(8):
+        for k in (0, 1):
+            plain = api.GBM3D_batch(imgs[k:k + 1], [25.0], o, use_graph=False)[0]
+            assert torch.equal(plain, captured[k])
