@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(128, OCC) k_match_video_bound(VideoMatchArgs A
     const uint32_t s = sel[k];
     const int a = (int)(s % D), b = (int)((s / D) % D), f = (int)(s / DD);
     A.volume[(size_t)(i * D + r) + (size_t)A.m * (j * D + c) + mn * k] =
-        A.pads[f][(size_t)(i * D + a + r) + (size_t)(j * D + b + c) * A.P];
+        __ldg(A.pads[f] + (size_t)(i * D + a + r) + (size_t)(j * D + b + c) * A.P);  // address from shared memory
   }
 }
 
