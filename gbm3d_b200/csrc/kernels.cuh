@@ -125,13 +125,19 @@ struct WaveletBank {
 struct LevelBands {
   float tau[8];  // hard threshold per band code (code 0 unused)
 };
+// One launch for n cycle spins: the distances in floats between one spin's arrays
+// and the next one's (analysis input or synthesis bands, approximation, output).
+struct SpinSet {
+  int n = 1;
+  size_t in = 0, approx = 0, out = 0;
+};
 // Analysis of one level + hard threshold.  in: Ly x Lx x Lz, read at
 // ((y-shift) mod Ly, (x-shift) mod Lx, (z-shift) mod Lz).  out: 8 bands, band
 // code fy + 2 fx + 4 fz, each (Ly/2)(Lx/2)(Lz/2) floats.
 // qcols: the coefficient columns (of Lx / 2) to produce.
 cudaError_t launch_wav_analysis(const float* in, int Ly, int Lx, int Lz, int shift, float* out,
                                 const WaveletBank& bk, const LevelBands& th, cudaStream_t st,
-                                const ColRange& qcols = ColRange());
+                                const ColRange& qcols = ColRange(), const SpinSet& spins = SpinSet());
 // Synthesis of one level: bands (codes 1..7) + approx -> out (Oy x Ox x Oz).
 // mode 0: out[p] = v; with shift_out, the value for p lands at p - shift_out.
 // Level-1 cycle-spin accumulation: first (store) / middle (add) / last
@@ -153,7 +159,7 @@ struct SynthOut {
 // cols: the output columns (values computed for p, before the shift) to produce.
 cudaError_t launch_wav_synthesis(const float* bands, const float* approx, int Oy, int Ox, int Oz,
                                  const SynthOut& o, const WaveletBank& bk, cudaStream_t st,
-                                 const ColRange& cols = ColRange());
+                                 const ColRange& cols = ColRange(), const SpinSet& spins = SpinSet());
 // medfilt3 of the volume (filtType 'median').
 cudaError_t launch_medfilt3(const float* V, int m, int n, int K, float* out, cudaStream_t st);
 // Aggregation weight 1/(TV(group)+eps) per group of Vavg (image-shaped, or

@@ -287,7 +287,7 @@ template <int LL, int H0, int HN, bool EVEN>
 __global__ void __launch_bounds__(32 * MW, 4) k_wav_analysis_march(const float* __restrict__ in, int Ly, int Lx,
                                                                    int Lz, int shift, float* __restrict__ out,
                                                                    FastBank fb, LevelBands th, int ty, int x_lo,
-                                                                   int x_len, int seg) {
+                                                                   int x_len, int seg, SpinSet sp) {
   begin_after_previous(in);
   constexpr int W = imax(LL, H0 + HN), HX = W / 2 - 1, HL = EVEN ? W / 2 : W / 2 - 1;
   constexpr int U = W > 2 ? W / 2 : 4, PD = 3;
@@ -295,8 +295,15 @@ __global__ void __launch_bounds__(32 * MW, 4) k_wav_analysis_march(const float* 
   __shared__ float2 sb[MW][2][4][32 + HL];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int Oy = Ly >> 1, Ox = Lx >> 1, Oz = Lz >> 1;
-  const int sgi = blockIdx.y, qz = blockIdx.z, strip = blockIdx.x * MW + warp;
+  const int sgi = blockIdx.y, strip = blockIdx.x * MW + warp;
   if (strip >= ty) return;
+  int qz = blockIdx.z;
+  if (sp.n > 1) {
+    const int spin = qz / Oz;
+    qz -= spin * Oz;
+    in += spin * sp.in;
+    out += spin * sp.out;
+  }
   const int q = strip * (32 - HL) - HL + lane;
   const bool live = lane >= HL && q < Oy;
   const size_t plane = (size_t)Ly * Lx;
@@ -416,15 +423,23 @@ template <int S0, int SN, int SH, bool RMW, bool PAIR>
 __global__ void __launch_bounds__(32 * MW, 4) k_wav_synthesis_march(const float* __restrict__ bands,
                                                                  const float* __restrict__ approx, int Oy, int Ox,
                                                                  int Oz, SynthOut o, FastBank fb, int ty, int x_lo,
-                                                                 int x_len, int seg) {
+                                                                 int x_len, int seg, SpinSet sp) {
   begin_after_previous(bands, approx);
   constexpr int W = imax(S0 + SN, SH), HS = W / 2, RW = HS + 1, NST = 4, PQ = 40;
   static_assert(W % 2 == 0 && 32 + HS <= PQ && 8 * HS <= 64, "ring");
   __shared__ float ring[MW][NST][8][PQ];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int Iy = Oy >> 1, Ix = Ox >> 1, Iz = Oz >> 1;
-  const int sgi = blockIdx.y, qz = blockIdx.z, strip = blockIdx.x * MW + warp;
+  const int sgi = blockIdx.y, strip = blockIdx.x * MW + warp;
   if (strip >= ty) return;
+  int qz = blockIdx.z;
+  if (sp.n > 1) {
+    const int spin = qz / Iz;
+    qz -= spin * Iz;
+    bands += spin * sp.in;
+    approx += spin * sp.approx;
+    o.out += spin * sp.out;
+  }
   const int q0 = strip * 32, q = q0 + lane;
   const bool live = q < Iy;
   const size_t bsz = (size_t)Iy * Ix * Iz, zoff = (size_t)Iy * Ix * qz;
@@ -629,25 +644,27 @@ static int march_segment(int len, long strips) {
 
 template <int LL, int H0, int HN>
 static cudaError_t launch_analysis_march(const float* in, int Ly, int Lx, int Lz, int shift, float* out,
-                                         const FastBank& fb, const LevelBands& th, cudaStream_t st, int lo, int len) {
+                                         const FastBank& fb, const LevelBands& th, cudaStream_t st, int lo, int len,
+                                         const SpinSet& sp) {
   const bool even = (shift & 1) == 0;
   const int nout = 32 - (imax(LL, H0 + HN) / 2 - (even ? 0 : 1));
-  const int ty = (Ly / 2 + nout - 1) / nout, seg = march_segment(len, (long)ty * (Lz / 2));
-  const dim3 grid((ty + MW - 1) / MW, (len + seg - 1) / seg, Lz / 2);
+  const int ty = (Ly / 2 + nout - 1) / nout, seg = march_segment(len, (long)ty * (Lz / 2) * sp.n);
+  const dim3 grid((ty + MW - 1) / MW, (len + seg - 1) / seg, Lz / 2 * sp.n);
   auto kern = even ? k_wav_analysis_march<LL, H0, HN, true> : k_wav_analysis_march<LL, H0, HN, false>;
-  launch_next(kern, grid, 32 * MW, 0, st, in, Ly, Lx, Lz, shift, out, fb, th, ty, lo, len, seg);
+  launch_next(kern, grid, 32 * MW, 0, st, in, Ly, Lx, Lz, shift, out, fb, th, ty, lo, len, seg, sp);
   return cudaGetLastError();
 }
 
 template <int S0, int SN, int SH>
 static cudaError_t launch_synthesis_march(const float* bands, const float* approx, int Oy, int Ox, int Oz,
-                                          const SynthOut& o, const FastBank& fb, cudaStream_t st, int lo, int len) {
-  const int ty = (Oy / 2 + 31) / 32, seg = march_segment(len, (long)ty * (Oz / 2));
-  const dim3 grid((ty + MW - 1) / MW, (len + seg - 1) / seg, Oz / 2);
+                                          const SynthOut& o, const FastBank& fb, cudaStream_t st, int lo, int len,
+                                          const SpinSet& sp) {
+  const int ty = (Oy / 2 + 31) / 32, seg = march_segment(len, (long)ty * (Oz / 2) * sp.n);
+  const dim3 grid((ty + MW - 1) / MW, (len + seg - 1) / seg, Oz / 2 * sp.n);
   const bool pair = (o.shift & 1) == 0;
   auto kern = o.first ? (pair ? k_wav_synthesis_march<S0, SN, SH, false, true> : k_wav_synthesis_march<S0, SN, SH, false, false>)
                       : (pair ? k_wav_synthesis_march<S0, SN, SH, true, true> : k_wav_synthesis_march<S0, SN, SH, true, false>);
-  launch_next(kern, grid, 32 * MW, 0, st, bands, approx, Oy, Ox, Oz, o, fb, ty, lo, len, seg);
+  launch_next(kern, grid, 32 * MW, 0, st, bands, approx, Oy, Ox, Oz, o, fb, ty, lo, len, seg, sp);
   return cudaGetLastError();
 }
 
@@ -775,15 +792,15 @@ static bool march_fits(int kind, int Ly, int Lx, int Lz) {
 
 cudaError_t launch_wav_analysis(const float* in, int Ly, int Lx, int Lz, int shift, float* out,
                                 const WaveletBank& bk, const LevelBands& th, cudaStream_t st,
-                                const ColRange& qcols) {
+                                const ColRange& qcols, const SpinSet& sp) {
   const int kind = fast_kind(bk);
   if (march_fits(kind, Ly, Lx, Lz)) {
     const FastBank fb = fast_bank(bk);
     const int O = Lx / 2, lo = qcols.all(O) ? 0 : pmod(qcols.lo, O), len = qcols.all(O) ? O : qcols.len;
     if (len == 0) return cudaSuccess;
-    if (kind == 1) return launch_analysis_march<10, 4, 2>(in, Ly, Lx, Lz, shift, out, fb, th, st, lo, len);
-    if (kind == 2) return launch_analysis_march<2, 0, 2>(in, Ly, Lx, Lz, shift, out, fb, th, st, lo, len);
-    return launch_analysis_march<8, 0, 8>(in, Ly, Lx, Lz, shift, out, fb, th, st, lo, len);
+    if (kind == 1) return launch_analysis_march<10, 4, 2>(in, Ly, Lx, Lz, shift, out, fb, th, st, lo, len, sp);
+    if (kind == 2) return launch_analysis_march<2, 0, 2>(in, Ly, Lx, Lz, shift, out, fb, th, st, lo, len, sp);
+    return launch_analysis_march<8, 0, 8>(in, Ly, Lx, Lz, shift, out, fb, th, st, lo, len, sp);
   }
   const size_t sm = analysis_smem(bk.reach_a);
   cudaError_t e = cudaFuncSetAttribute(k_wav_analysis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -792,13 +809,14 @@ cudaError_t launch_wav_analysis(const float* in, int Ly, int Lx, int Lz, int shi
   tile_span(qcols, Lx / 2, TQ, t0, nt);
   if (nt == 0) return cudaSuccess;
   dim3 grid((Ly / 2 + TQ - 1) / TQ, nt, Lz / 2);
-  k_wav_analysis<<<grid, 256, sm, st>>>(in, Ly, Lx, Lz, shift, out, bk, th, t0);
+  for (int q = 0; q < sp.n; ++q)
+    k_wav_analysis<<<grid, 256, sm, st>>>(in + q * sp.in, Ly, Lx, Lz, shift, out + q * sp.out, bk, th, t0);
   return cudaGetLastError();
 }
 
 cudaError_t launch_wav_synthesis(const float* bands, const float* approx, int Oy, int Ox, int Oz,
                                  const SynthOut& o, const WaveletBank& bk, cudaStream_t st,
-                                 const ColRange& cols) {
+                                 const ColRange& cols, const SpinSet& sp) {
   const int kind = fast_kind(bk);
   if (march_fits(kind, Oy, Ox, Oz)) {
     const FastBank fb = fast_bank(bk);
@@ -807,9 +825,9 @@ cudaError_t launch_wav_synthesis(const float* bands, const float* approx, int Oy
     const int pairs = cols.all(Ox) ? I : cols.len == 0 ? 0 : (pmod(cols.lo, Ox) + cols.len - 1) / 2 - first + 1;
     const int lo = pairs >= I ? 0 : first, len = pairs >= I ? I : pairs;
     if (len == 0) return cudaSuccess;
-    if (kind == 1) return launch_synthesis_march<4, 2, 10>(bands, approx, Oy, Ox, Oz, o, fb, st, lo, len);
-    if (kind == 2) return launch_synthesis_march<0, 2, 2>(bands, approx, Oy, Ox, Oz, o, fb, st, lo, len);
-    return launch_synthesis_march<0, 8, 8>(bands, approx, Oy, Ox, Oz, o, fb, st, lo, len);
+    if (kind == 1) return launch_synthesis_march<4, 2, 10>(bands, approx, Oy, Ox, Oz, o, fb, st, lo, len, sp);
+    if (kind == 2) return launch_synthesis_march<0, 2, 2>(bands, approx, Oy, Ox, Oz, o, fb, st, lo, len, sp);
+    return launch_synthesis_march<0, 8, 8>(bands, approx, Oy, Ox, Oz, o, fb, st, lo, len, sp);
   }
   const size_t sm = synthesis_smem(bk.reach_s);
   cudaError_t e = cudaFuncSetAttribute(k_wav_synthesis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -818,7 +836,11 @@ cudaError_t launch_wav_synthesis(const float* bands, const float* approx, int Oy
   tile_span(cols, Ox, TP, t0, nt);
   if (nt == 0) return cudaSuccess;
   dim3 grid((Oy + TP - 1) / TP, nt, Oz / 2);
-  k_wav_synthesis<<<grid, 256, sm, st>>>(bands, approx, Oy, Ox, Oz, o, bk, t0);
+  for (int q = 0; q < sp.n; ++q) {
+    SynthOut oq = o;
+    oq.out += q * sp.out;
+    k_wav_synthesis<<<grid, 256, sm, st>>>(bands + q * sp.in, approx + q * sp.approx, Oy, Ox, Oz, oq, bk, t0);
+  }
   return cudaGetLastError();
 }
 
