@@ -105,6 +105,7 @@ T* buf(gbm3d_ctx* c, const char* cname, size_t count) {
   auto it = c->bufs.find(name);
   if (it != c->bufs.end() && it->second.second >= bytes) return reinterpret_cast<T*>(it->second.first);
   if (it != c->bufs.end()) {
+    c->graph_key.clear();  // a captured graph may hold the old address: capture again
     cudaFree(it->second.first);
     c->bufs.erase(it);
   }

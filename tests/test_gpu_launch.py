@@ -21,3 +21,22 @@ def test_overlapped_launches_equal_captured(gpu, m, n, s):
         for k in (0, 1):
             plain = api.GBM3D_batch(imgs[k:k + 1], [25.0], o, use_graph=False)[0]
             assert torch.equal(plain, captured[k])
+
+
+@pytest.mark.parametrize("first,between", [((96, 80), (160, 128)), ((320, 256), (304, 256))])
+def test_graph_replay_after_buffers_grew(gpu, first, between):
+    """A call in between that needs larger workspaces: the batch is captured again."""
+    import torch
+    from gbm3d_b200 import api
+    from gbm3d_b200._lib import Context
+    ctx = Context(0)
+    o = options.resolve_opts({"profile": "default"})
+    x, y = [torch.from_numpy(np.ascontiguousarray(synth.noisy_image(m, n, 25.0, seed=m)[1].T)).cuda()
+            for m, n in (first, between)]
+    out = [torch.empty_like(x)]
+    want = api.GBM3D_batch([x], [25.0], o, ctx=ctx, use_graph=True, outputs=out)[0].clone()
+    for _ in range(2):  # a replay, then the call after the workspaces grew
+        out[0].zero_()
+        api.GBM3D_batch([x], [25.0], o, ctx=ctx, use_graph=True, outputs=out)
+        assert torch.equal(out[0], want)
+        api.GBM3D_batch([y], [25.0], o, ctx=ctx, use_graph=False)
