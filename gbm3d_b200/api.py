@@ -262,8 +262,8 @@ def GBM3D(I, sigma, opts: dict | None = None, ctx: Context | None = None):
     I = np.asfortranarray(I, dtype=np.float64)
     m, n = I.shape
     o = _opt.resolve_opts(opts, shape=(m, n), sigma=sigma)
-    U = np.zeros((m, n), order="F")
-    U1 = np.zeros((m, n), order="F")
+    U = np.empty((m, n), order="F")
+    U1 = np.empty((m, n), order="F")
     co = c_opts(o)
     sg = np.asarray(sigma, dtype=np.float64)
     if sg.ndim >= 1 and sg.shape[0] > 1:

@@ -8,6 +8,8 @@
 // denoiseAndAggregateWieFast, denoiseAndAggregateWie) copy their host
 // arguments in and their results out, so a MEX gateway can call them with
 // mxArray data directly.
+#include <sys/mman.h>
+
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -53,6 +55,7 @@ struct gbm3d_ctx {
   // order the copies of a slot with the compute that uses it
   cudaStream_t h2d = nullptr, d2h = nullptr;
   cudaEvent_t in_ready[2] = {}, in_free[2] = {}, out_ready[2] = {}, out_free[2] = {};
+  cudaEvent_t step1_done = nullptr;
   int slot = 0;
   bool async_pending = false;
   int* sticky = nullptr;  // OR of the status words of the asynchronous calls since the last synchronisation
@@ -1002,11 +1005,12 @@ int padded_size(const gbm3d_opts* o, int L, int d, int dw, int st1, int st2) {
 // tau_in (levels x 7) and sigwie_in (blockSizeWie^2) replace sigma * getTau
 // and the scalar Wiener sigma on the coloured-noise path (GBM3D.m:30-36);
 // sigma is then what the matchers use, mean(sqrt(sigmaPSD)).
+// step1_done: recorded once dU1 is written and step 2 is still to come.
 // strip (c_lo < c_hi): only output columns [c_lo, c_hi) of dU are exact (the
 // strip form); the rest of dU holds whatever the restricted stages left there.
 void pipeline(gbm3d_ctx* c, const double* dI, int m, int n, double sigma, const gbm3d_opts* o, double* dU,
               double* dU1, const double* tau_in = nullptr, const double* sigwie_in = nullptr, int c_lo = 0,
-              int c_hi = 0) {
+              int c_hi = 0, cudaEvent_t step1_done = nullptr) {
   check_opts(c, o);
   int d, dw, d2, K;
   opts_dims(o, d, dw, d2, K);
@@ -1110,6 +1114,7 @@ void pipeline(gbm3d_ctx* c, const double* dI, int m, int n, double sigma, const 
   if (!o->Wiener) return;
   }
 
+  if (step1_done) ck(c, cudaEventRecord(step1_done, c->st), "cudaEventRecord");
   // step 2: empirical Wiener estimate over the Wiener match spins
   const int M2 = grid_count(Mp, dw, st2), N2 = grid_count(Np, dw, st2);
   uint32_t* S2 = buf<uint32_t>(c, "p.S2", (size_t)K * M2 * N2);
@@ -1195,6 +1200,7 @@ void gbm3d_ctx_destroy(gbm3d_ctx* c) {
     for (int k = 0; k < 2; ++k)
       for (cudaEvent_t e : {c->in_ready[k], c->in_free[k], c->out_ready[k], c->out_free[k]})
         if (e) cudaEventDestroy(e);
+    if (c->step1_done) cudaEventDestroy(c->step1_done);
   }
   if (c->sticky) cudaFree(c->sticky);
   if (c->tc_hist) cudaFree(c->tc_hist);
@@ -2315,6 +2321,33 @@ int gbm3d_strip_work(const gbm3d_opts* o, int m, int n, int col_lo, int col_hi, 
   }
 }
 
+// The copy streams of the host-buffer calls and their events, made at the first such call.
+static void copy_streams(gbm3d_ctx* c) {
+  if (c->h2d) return;
+  ck(c, cudaStreamCreateWithFlags(&c->h2d, cudaStreamNonBlocking), "cudaStreamCreate");
+  ck(c, cudaStreamCreateWithFlags(&c->d2h, cudaStreamNonBlocking), "cudaStreamCreate");
+  for (int k = 0; k < 2; ++k)
+    for (cudaEvent_t* e : {&c->in_ready[k], &c->in_free[k], &c->out_ready[k], &c->out_free[k]})
+      ck(c, cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
+  ck(c, cudaEventCreateWithFlags(&c->step1_done, cudaEventDisableTiming), "cudaEventCreate");
+  ck(c, cudaMalloc(&c->sticky, sizeof(int)), "cudaMalloc");
+  ck(c, cudaMemset(c->sticky, 0, sizeof(int)), "cudaMemset");
+}
+
+// Makes every page of a host array present, its contents as they are (a request
+// that the kernel cannot fulfil changes nothing).
+static void populate_pages(double* p, size_t bytes) {
+  const uintptr_t from = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)4095;
+  const uintptr_t to = (reinterpret_cast<uintptr_t>(p) + bytes + 4095) & ~(uintptr_t)4095;
+  constexpr int POPULATE_WRITE = 23;  // MADV_POPULATE_WRITE, Linux 5.14
+  madvise(reinterpret_cast<void*>(from), to - from, POPULATE_WRITE);
+}
+
+// The host's part of the copies runs under the kernels: outputs that the caller has just
+// allocated get their pages while step 1 runs (inside the copies each page is a
+// fault: 1.8 instead of 1.0 ms for a 512 x 512 call whenever the allocator hands out new
+// ones), and U1 is copied on its own stream while step 2 runs.  512 x 512 from pageable
+// arrays 0.99 -> 0.86 ms, new pages or not.
 static int denoise_host(gbm3d_ctx* c, const double* I, int m, int n, double sigma, const gbm3d_opts* o, double* U,
                         double* U1, const double* tau, const double* sigwie) {
   return guarded(c, [&] {
@@ -2324,12 +2357,22 @@ static int denoise_host(gbm3d_ctx* c, const double* I, int m, int n, double sigm
     double* dI = buf<double>(c, "h.I", px);
     double* dU = buf<double>(c, "h.U", px);
     double* dU1 = U1 ? buf<double>(c, "h.U1", px) : nullptr;
+    // one array given for both estimates ends as U1: then the copies stay in that order
+    const bool early = U1 && o && o->Wiener && (U1 + px <= U || U + px <= U1);
+    if (early) copy_streams(c);
     ck(c, cudaMemcpyAsync(dI, I, px * 8, cudaMemcpyHostToDevice, c->st), "H2D");
-    pipeline(c, dI, m, n, sigma, o, dU, dU1, tau, sigwie);
+    pipeline(c, dI, m, n, sigma, o, dU, dU1, tau, sigwie, 0, 0, early ? c->step1_done : nullptr);
+    if (U1) populate_pages(U1, px * 8);
+    populate_pages(U, px * 8);
+    if (early) {
+      ck(c, cudaStreamWaitEvent(c->d2h, c->step1_done, 0), "cudaStreamWaitEvent");
+      ck(c, cudaMemcpyAsync(U1, dU1, px * 8, cudaMemcpyDeviceToHost, c->d2h), "D2H");
+    }
     ck(c, cudaMemcpyAsync(U, dU, px * 8, cudaMemcpyDeviceToHost, c->st), "D2H");
-    if (U1) ck(c, cudaMemcpyAsync(U1, dU1, px * 8, cudaMemcpyDeviceToHost, c->st), "D2H");
+    if (U1 && !early) ck(c, cudaMemcpyAsync(U1, dU1, px * 8, cudaMemcpyDeviceToHost, c->st), "D2H");
     int flag = 0;
     ck(c, cudaMemcpyAsync(&flag, c->flag, sizeof(int), cudaMemcpyDeviceToHost, c->st), "D2H");
+    if (early) ck(c, cudaStreamSynchronize(c->d2h), "sync");
     ck(c, cudaStreamSynchronize(c->st), "sync");
     report_flag(c, flag);
   });
@@ -2345,15 +2388,7 @@ int gbm3d_denoise_async(gbm3d_ctx* c, const double* I, int m, int n, double sigm
   return guarded(c, [&] {
     if (!I || !U || !o) argfail(c, "missing argument");
     if (m < 1 || n < 1 || m > 32000 || n > 32000) argfail(c, "image size out of range");
-    if (!c->h2d) {
-      ck(c, cudaStreamCreateWithFlags(&c->h2d, cudaStreamNonBlocking), "cudaStreamCreate");
-      ck(c, cudaStreamCreateWithFlags(&c->d2h, cudaStreamNonBlocking), "cudaStreamCreate");
-      for (int k = 0; k < 2; ++k)
-        for (cudaEvent_t* e : {&c->in_ready[k], &c->in_free[k], &c->out_ready[k], &c->out_free[k]})
-          ck(c, cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
-      ck(c, cudaMalloc(&c->sticky, sizeof(int)), "cudaMalloc");
-      ck(c, cudaMemset(c->sticky, 0, sizeof(int)), "cudaMemset");
-    }
+    copy_streams(c);
     const size_t px = (size_t)m * n;
     const int k = c->slot;
     double* dI = buf<double>(c, k ? "a.I1" : "a.I0", px);

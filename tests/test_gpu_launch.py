@@ -40,3 +40,30 @@ def test_graph_replay_after_buffers_grew(gpu, first, between):
         api.GBM3D_batch([x], [25.0], o, ctx=ctx, use_graph=True, outputs=out)
         assert torch.equal(out[0], want)
         api.GBM3D_batch([y], [25.0], o, ctx=ctx, use_graph=False)
+
+
+@pytest.mark.parametrize("m,n", [(24, 24), (65, 47), (301, 203)])
+def test_host_arrays_shared_between_arguments(gpu, m, n):
+    """The host call's copies: outputs in one array (it ends as U1), in place, and apart."""
+    import ctypes as C
+    from gbm3d_b200 import api
+    from gbm3d_b200._lib import lib
+    o = options.resolve_opts({"profile": "default"})
+    o.update(blockSize=8, blockSizeWie=8, matchSize=24, refStride=8, refStrideWie=8)
+    x = np.asfortranarray(synth.noisy_image(m, n, 25.0, seed=3)[1])
+    U, out = api.GBM3D(x, 25.0, o)
+    co, ctx = api.c_opts(o), api.context()
+    p = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
+
+    def call(I, u, u1):
+        ctx.check(lib().gbm3d_denoise(ctx.h, p(I), m, n, 25.0, C.byref(co), p(u), p(u1)))
+
+    both = np.zeros((m, n), order="F")
+    call(x, both, both)
+    assert np.array_equal(both, out["U1"])
+    inplace, u1 = x.copy(order="F"), np.zeros((m, n), order="F")
+    call(inplace, inplace, u1)
+    assert np.array_equal(inplace, U) and np.array_equal(u1, out["U1"])
+    u, inplace = np.zeros((m, n), order="F"), x.copy(order="F")
+    call(inplace, u, inplace)
+    assert np.array_equal(u, U) and np.array_equal(inplace, out["U1"])
