@@ -278,9 +278,14 @@ static cudaError_t launch_px_cap(const AggArgs& A, cudaStream_t st) {
 //   PT, the region's column pitch, is 8 modulo 16 pixels of eight bytes: the
 // 8 x 4 pixels of a half patch fall on distinct banks at every block offset.
 //   The warp enumerates the candidates (reference i, j, slot k) whose search
-// window reaches its region, in loop order, and needs no barrier.  A block is
+// window reaches its region, in loop order.  A block is
 // 256 (1024) contiguous bytes (group-major), two lines where the image-shaped
 // volume has eight, and is prefetched into L2 when it is listed.
+//   A region of 8 x 8 runs where the GPU is not full (301 x 203: 1.7 warps per
+// scheduler, each issuing one instruction in seven cycles), so there a second warp makes
+// list r + 1 while the first walks list r: 322 -> 278 us for the four launches of
+// 301 x 203.  On the larger regions the second warp takes slots from other regions
+// (16 x 16: 512^2 126 -> 168 us; 24 x 24: 4096^2 1.15 -> 1.81 ms).
 //   Bounds at 1024^2 dense (ncu): shared-memory pipe 61 %, issue 42-50 %, DRAM
 // 33 %; 272 us per launch against 625 us pixel at a time (of which the
 // group-major layout with its prefetch 310: DRAM reads 2.07 -> 0.72 GB).
@@ -298,14 +303,17 @@ struct AggBlk {
   static constexpr int COLS = RC + 2 * D - 1;
   static constexpr int SV = KAHAN ? 4 : 2;  // floats per pixel: u, w (and their compensations)
   static constexpr int NB = D == 8 ? 8 : 4; // entries loaded together
-    static constexpr int EB = 4;              // candidates per lane and enumeration round
-  static constexpr int LC = 2 * 32 * EB;    // list capacity
-  static constexpr size_t BYTES = (size_t)(LC + 2 * NB) * sizeof(int4) + (size_t)PT * COLS * SV * sizeof(float);
+  static constexpr int EB = 4;              // candidates per lane and enumeration round
+  static constexpr bool TWO = RR <= 8;      // one warp lists, the other walks
+  static constexpr int NT = TWO ? 64 : 32;
+  static constexpr int LC = (TWO ? 96 : 128) + 32 * EB;  // list capacity
+  static constexpr int LISTS = (TWO ? 2 : 1) * (LC + 2 * NB);
+  static constexpr size_t BYTES = (size_t)LISTS * sizeof(int4) + (size_t)PT * COLS * SV * sizeof(float);
   static_assert(PT >= RR + 2 * D - 1, "pitch");
 };
 
 template <int D, int D2, bool WIE, bool KAHAN, int RR, int RC>
-__global__ void __launch_bounds__(32) k_aggregate_blk(AggArgs A) {
+__global__ void __launch_bounds__(AggBlk<D, KAHAN, RR, RC>::NT) k_aggregate_blk(AggArgs A) {
   const float* blocks = A.blocks;
   const float* gw = A.gw;
   const uint32_t* Sg = A.S;
@@ -316,11 +324,12 @@ __global__ void __launch_bounds__(32) k_aggregate_blk(AggArgs A) {
   constexpr int NP = D * D / 32, CSTEP = 32 / D;  // pixels per lane, block columns between them
   constexpr int H = D2 / 2;
   extern __shared__ int4 smv[];
-  const int lane = threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const bool walks = !G::TWO || threadIdx.x < 32, lists = !G::TWO || threadIdx.x >= 32;
   int4* lst = smv;
-  float* acc = reinterpret_cast<float*>(smv + G::LC + 2 * NB);
+  float* acc = reinterpret_cast<float*>(smv + G::LISTS);
   const unsigned FULL = 0xffffffffu, below = (1u << lane) - 1u;
-  for (int e = lane; e < PT * G::COLS * SV / 4; e += 32) reinterpret_cast<float4*>(acc)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int e = threadIdx.x; e < PT * G::COLS * SV / 4; e += G::NT) reinterpret_cast<float4*>(acc)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
 
   const int tiles_r = (A.m + RR - 1) / RR, tiles_c = (A.n + RC - 1) / RC;
   const int tcol = (int)(blockIdx.x / tiles_r) + A.ct0;  // the window's column tiles, modulo the count
@@ -439,40 +448,61 @@ __global__ void __launch_bounds__(32) k_aggregate_blk(AggArgs A) {
       C.gw[u] = WIE ? 0.f : __ldg(gw + g);
     }
   };
-  __syncwarp();
-  int cnt = 0;
+  // the entries of candidates base, base + 1, ... until the list may be full
+  int base = 0;
   Cand next;
-  if (total > 0) look(next, 0);
-  for (int base = 0; base < total; base += 32 * EB) {
-    const Cand cur = next;
-    if (base + 32 * EB < total) look(next, base + 32 * EB);
+  if (lists && total > 0) look(next, 0);
+  auto fill = [&]() {
+    int cnt = 0;
+    for (; base < total && cnt <= G::LC - 32 * EB; base += 32 * EB) {
+      const Cand cur = next;
+      if (base + 32 * EB < total) look(next, base + 32 * EB);
 #pragma unroll
-    for (int u = 0; u < EB; ++u) {
-      int i, j, k;
-      decode(min(base + 32 * u + lane, total - 1), i, j, k);
-      const int e = cur.e[u], r0 = i * s + e % D2 - PR0, c0 = j * s + e / D2 - PC0;
-      const bool hit = base + 32 * u + lane < total && k < cur.nm[u] && r0 > -D && r0 < RR && c0 > -D && c0 < RC;
-      const unsigned bal = __ballot_sync(FULL, hit);
-      if (hit) {
-        const int g = i + A.M * j;
-        int4 en;
-        en.x = (r0 + D + PT * (c0 + D)) * SV;
-        en.y = (g * K + k) * (D * D);
-        en.z = WIE ? g * (D * D) : __float_as_int(cur.gw[u]);
-        en.w = 0;
-        lst[cnt + __popc(bal & below)] = en;
-        prefetch_l2<D * D>(blocks + (size_t)(unsigned)en.y);
+      for (int u = 0; u < EB; ++u) {
+        int i, j, k;
+        decode(min(base + 32 * u + lane, total - 1), i, j, k);
+        const int e = cur.e[u], r0 = i * s + e % D2 - PR0, c0 = j * s + e / D2 - PC0;
+        const bool hit = base + 32 * u + lane < total && k < cur.nm[u] && r0 > -D && r0 < RR && c0 > -D && c0 < RC;
+        const unsigned bal = __ballot_sync(FULL, hit);
+        if (hit) {
+          const int g = i + A.M * j;
+          int4 en;
+          en.x = (r0 + D + PT * (c0 + D)) * SV;
+          en.y = (g * K + k) * (D * D);
+          en.z = WIE ? g * (D * D) : __float_as_int(cur.gw[u]);
+          en.w = 0;
+          lst[cnt + __popc(bal & below)] = en;
+          prefetch_l2<D * D>(blocks + (size_t)(unsigned)en.y);
+        }
+        cnt += __popc(bal);
       }
-      cnt += __popc(bal);
     }
-    if (cnt > G::LC - 32 * EB) {
-      walk(cnt);
-      cnt = 0;
+    return cnt;
+  };
+  if constexpr (G::TWO) {
+    // list r + 1 is made while list r is walked; one barrier per list
+    __shared__ int scnt[2];
+    for (int r = 0;; ++r) {
+      lst = smv + (r & 1) * (G::LC + 2 * NB);
+      if (lists) {
+        const int cnt = fill();
+        if (lane == 0) scnt[r & 1] = base < total ? cnt : -1 - cnt;  // negative: the last one
+      }
+      __syncthreads();
+      const int c = scnt[r & 1], cnt = c < 0 ? -1 - c : c;
+      if (walks && cnt) walk(cnt);
+      if (c < 0) break;
     }
+    __syncthreads();
+  } else {
+    __syncwarp();
+    while (base < total) {
+      const int cnt = fill();
+      if (cnt) walk(cnt);
+    }
+    __syncwarp();
   }
-  if (cnt) walk(cnt);
-  __syncwarp();
-  for (int e = lane; e < RR * RC; e += 32) {
+  for (int e = threadIdx.x; e < RR * RC; e += G::NT) {
     const int r = e % RR, c = e / RR, orow = R0 + r, ocol = C0 + c;
     if (orow < A.m && ocol < A.n) {
       const float2 v = *reinterpret_cast<const float2*>(acc + (r + D + PT * (c + D)) * SV);
@@ -492,7 +522,8 @@ static cudaError_t launch_blk(const AggArgs& A, cudaStream_t st) {
   int nt;
   tile_span(A.cols, A.n, RC, B.ct0, nt);
   if (nt == 0) return cudaSuccess;
-  launch_next(k_aggregate_blk<D, D2, WIE, KAHAN, RR, RC>, ((A.m + RR - 1) / RR) * nt, 32, sm, st, B);
+  launch_next(k_aggregate_blk<D, D2, WIE, KAHAN, RR, RC>, ((A.m + RR - 1) / RR) * nt,
+              AggBlk<D, KAHAN, RR, RC>::NT, sm, st, B);
   return cudaGetLastError();
 }
 
@@ -502,9 +533,9 @@ static cudaError_t launch_blk(const AggArgs& A, cudaStream_t st) {
 // regions per SM on, 16 x 16 from 5, else 8 x 8.  Smaller regions touch more
 // entries per pixel (at stride 8: 0.42 per pixel at 24, 0.52 at 16, 0.88 at 8) but
 // fill the GPU.  Measured, all aggregations of a call in us (pixel-at-a-time
-// kernel / 24 / 16 / 8): 4096^2 at strides 8 / 7 2232 / 1177 / 1394 / 2791; 1024^2 dense
-// 2502 / 1190 / 1340 / 2042; 512^2 reference tiling 131 / 146 / 125 / 175; 301 x 203 dense
-// 590 / 730 / 465 / 318; 128 x 96 77 / 106 / 82 / 69.
+// kernel / 24 / 16 / 8 with one warp): 4096^2 at strides 8 / 7 2232 / 1177 / 1394 / 2791; 1024^2
+// dense 2502 / 1190 / 1340 / 2042; 512^2 reference tiling 131 / 146 / 125 / 175; 301 x 203
+// dense 590 / 730 / 465 / 318 (two warps 278); 128 x 96 77 / 106 / 82 / 69 (67).
 // Otherwise (the median filter's image-shaped volume, other patches): pixel at
 // a time, with the list capacity from the expected entries of a tile:
 // (candidate references across the tile's reach) x K, about a quarter of which

@@ -58,3 +58,18 @@ def test_hard_threshold_aggregation(gpu, oracle, m, n, d, s, d2):
     U, W = gpu.denoiseAndAggregateGPU(V, _as_set(S, cnt), tau, Psi, Psi2, o)
     Uo, Wo = oracle.denoiseAndAggregateGPU(V, S, tau, o, cnt=cnt, filters=oracle.bior_filters(), prec=32)
     assert np.array_equal(U, Uo) and np.array_equal(W, Wo)
+
+
+@pytest.mark.parametrize("m,n,d,s,K", [(40, 33, 8, 1, 32), (48, 41, 16, 1, 16), (33, 32, 8, 8, 8)])
+def test_full_and_empty_lists(gpu, oracle, m, n, d, s, K):
+    """Every match at its own reference: rounds of candidates that all hit or all miss."""
+    rng = np.random.default_rng(m + n + K)
+    M, N = (m - d) // s + 1, (n - d) // s + 1
+    m, n = (M - 1) * s + d, (N - 1) * s + d
+    S = np.full((K, M, N), 32 * 16 + 17, dtype=np.uint32, order="F")
+    V1 = np.asfortranarray(rng.uniform(0, 255, (d, d, K, M, N)).astype(np.float32))
+    V2 = np.asfortranarray(V1 + 25 * rng.standard_normal(V1.shape).astype(np.float32))
+    o = _opts(d, s, K)
+    U, W = gpu.denoiseAndAggregateWieFast(V1, V2, _as_set(S), 25.0, o)
+    Uo, Wo = oracle.denoiseAndAggregateWieFast(V1, V2, S, 25.0, o, prec=32)
+    assert np.array_equal(U, Uo) and np.array_equal(W, Wo)
