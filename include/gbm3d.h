@@ -358,7 +358,9 @@ int gbm3d_stage_times(const gbm3d_ctx* ctx, float* ms, int n);
  * flight have landed, and the call reports GBM3D_ERR_CUDA ("... did not
  * complete within its wait limit").  A negative value is a probe of that
  * path: every CTA first waits, with the limit -cycles, on a barrier that
- * nothing completes, so the next matching call fails that way.  Not in the
+ * nothing completes, so the next matching call fails that way.  At search
+ * size 32 the forms run the bounded matcher unless a limit is set here or the
+ * statistics below are on (the match sets are the same).  Not in the
  * reference. */
 int gbm3d_ctx_set_tc_wait(gbm3d_ctx* ctx, long long cycles);
 
