@@ -2105,6 +2105,12 @@ void key_add(std::string& key, const T& v) {
   key.append(reinterpret_cast<const char*>(&v), sizeof(T));
 }
 
+// Context settings that the launch sequence of a batch depends on (run_match).
+void key_add_settings(std::string& key, const gbm3d_ctx* c) {
+  key_add(key, c->tc_wait);
+  key_add(key, c->tc_stats);
+}
+
 }  // namespace
 
 extern "C" {
@@ -2120,6 +2126,7 @@ int gbm3d_denoise_batch(gbm3d_ctx* c, int nimg, const double* const* I, const in
     for (int k = 0; k < nimg; ++k) ord[k] = k;
     std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return (long)m[a] * n[a] > (long)m[b] * n[b]; });
     std::string key("batch");
+    key_add_settings(key, c);
     key_add(key, *o);
     for (int k = 0; k < nimg; ++k) {
       key_add(key, I[k]);
@@ -2164,6 +2171,7 @@ int gbm3d_denoise_mixed(gbm3d_ctx* c, const gbm3d_mixed_batch* b, const gbm3d_op
     for (int k = 0; k < b->n_grey; ++k) learned |= grey_o(k)->form == 2;
     for (int k = 0; k < b->n_rgb; ++k) learned |= rgb_o(k)->form == 2;
     std::string key("mixed");
+    key_add_settings(key, c);
     key_add(key, *o);
     if (b->video) key_add(key, *ov);
     key_add(key, (int)(b->grey_opts != nullptr));
