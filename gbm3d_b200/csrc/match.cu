@@ -310,7 +310,8 @@ __global__ void __launch_bounds__(256) k_gather_volume(const float* __restrict__
                                                        int K, const uint32_t* __restrict__ S,
                                                        const int32_t* __restrict__ cnt, float* __restrict__ vol) {
   begin_after_previous(pad, S, cnt);
-  const int y = blockIdx.x * 256 + threadIdx.x, x = blockIdx.y, vm = M * D;
+  // columns along x: a dense grid has more of them than the other grid dimensions hold
+  const int y = blockIdx.y * 256 + threadIdx.x, x = blockIdx.x, vm = M * D;
   if (y >= vm) return;
   const int i = y / D, r = y % D, j = x / D, c = x % D, h = d2 / 2;
   const size_t g = i + (size_t)M * j;
@@ -318,7 +319,7 @@ __global__ void __launch_bounds__(256) k_gather_volume(const float* __restrict__
   const uint32_t* Sg = S + g * K;
   const float* src = pad + (size_t)(i * s + r) + (size_t)(j * s + c) * P;
   float* dst = vol + y + (size_t)vm * x;
-  const size_t slot = (size_t)vm * gridDim.y;
+  const size_t slot = (size_t)vm * gridDim.x;
 #pragma unroll 8
   for (int k = 0; k < K; ++k) {
     int e = (int)__ldg(Sg + k) - 1;
@@ -330,8 +331,7 @@ __global__ void __launch_bounds__(256) k_gather_volume(const float* __restrict__
 
 cudaError_t launch_gather_volume(const float* pad, int P, int M, int N, int s, int d, int d2, int K, const uint32_t* S,
                                  const int32_t* cnt, float* vol, cudaStream_t st) {
-  const dim3 grid((M * d + 255) / 256, N * d);
-  if (N * d > 65535) return cudaErrorInvalidValue;
+  const dim3 grid(N * d, (M * d + 255) / 256);
   switch (d) {
     case 8: launch_next(k_gather_volume<8>, grid, 256, 0, st, pad, P, M, s, d2, K, S, cnt, vol); break;
     case 16: launch_next(k_gather_volume<16>, grid, 256, 0, st, pad, P, M, s, d2, K, S, cnt, vol); break;
