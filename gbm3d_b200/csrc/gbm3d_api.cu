@@ -591,7 +591,8 @@ float* run_wavelet_ht(gbm3d_ctx* c, const float* vol, int m, int n, int K, int l
   if (cycleSpin < 1) argfail(c, "cycleSpin must be >= 1");
   const size_t voxels = (size_t)m * n * K;
   const bool together = !w && levels > 1 && voxels * cycleSpin <= SPINS_TOGETHER;
-  const int copies = together ? cycleSpin : 1;
+  // spin s of a round of `copies`; the second level's slot pairs of all of them are one grid's z
+  const int copies = together ? std::min(cycleSpin, 65535 / (K >> 2)) : 1;
   std::vector<float*> coef(levels), rec(levels);
   std::vector<size_t> insz(levels);
   for (int lv = 0; lv < levels; ++lv) {
@@ -606,26 +607,25 @@ float* run_wavelet_ht(gbm3d_ctx* c, const float* vol, int m, int n, int K, int l
   }
   {
   StageTimer tw(c, 2);
-  // spins s .. s + count - 1 of a level
-  auto analyse = [&](int lv, int s, int count) {
+  // spins s .. s + count - 1 of a level, the first of them number `slot` of its round
+  auto analyse = [&](int lv, int s, int slot, int count) {
     SpinSet sp;
     sp.n = count;
     sp.in = lv == 0 ? 0 : insz[lv - 1];
     sp.out = insz[lv];
     const float* in = lv == 0 ? vol : coef[lv - 1];
-    float* out = coef[lv] + (together && lv == 0 ? s * insz[0] : 0);
+    float* out = coef[lv] + slot * insz[lv];
     launched(c, launch_wav_analysis(in, m >> lv, n >> lv, K >> lv, lv == 0 ? s : 0, out, bk, th[lv], c->st,
                                     w ? w->an[lv] : ColRange(), sp),
              "wav_analysis");
   };
-  auto synthesise = [&](int lv, int s, int count) {
+  auto synthesise = [&](int lv, int s, int slot, int count) {
     const bool top = lv == levels - 1;
     SpinSet sp;
     sp.n = count;
     sp.in = insz[lv];
     sp.approx = top ? insz[lv] : insz[lv + 1];
     sp.out = insz[lv];
-    const size_t own = together && lv == 0 ? s : 0;
     SynthOut o{};
     if (lv == 0) {
       o.out = vsum;
@@ -644,15 +644,16 @@ float* run_wavelet_ht(gbm3d_ctx* c, const float* vol, int m, int n, int K, int l
       o.last = 0;
       o.cycles = 1.f;
     }
-    launched(c, launch_wav_synthesis(coef[lv] + own * sp.in, (top ? coef[lv] : rec[lv + 1]) + own * sp.approx,
+    launched(c, launch_wav_synthesis(coef[lv] + slot * sp.in, (top ? coef[lv] : rec[lv + 1]) + slot * sp.approx,
                                      m >> lv, n >> lv, K >> lv, o, bk, c->st, w ? w->sy[lv] : ColRange(), sp),
              "wav_synthesis");
   };
   for (int s = 0; s < cycleSpin; s += copies) {
-    for (int q = 0; q < copies; ++q) analyse(0, s + q, 1);
-    for (int lv = 1; lv < levels; ++lv) analyse(lv, s, copies);
-    for (int lv = levels - 1; lv >= 1; --lv) synthesise(lv, s, copies);
-    for (int q = 0; q < copies; ++q) synthesise(0, s + q, 1);
+    const int count = std::min(copies, cycleSpin - s);
+    for (int q = 0; q < count; ++q) analyse(0, s + q, q, 1);
+    for (int lv = 1; lv < levels; ++lv) analyse(lv, s, 0, count);
+    for (int lv = levels - 1; lv >= 1; --lv) synthesise(lv, s, 0, count);
+    for (int q = 0; q < count; ++q) synthesise(0, s + q, q, 1);
   }
   }
   }
