@@ -569,12 +569,15 @@ struct Spin2Cols {
 };
 
 // The levels below the first are the same for every cycle spin but for their input, so
-// the spins of a volume up to this many voxels, all spins counted, share those launches
-// (each spin keeps its coefficients, at most 0.5 GB more).  Eight launches fewer for each pair of
-// three-level volumes: 128 x 96 242 -> 209 us, 301 x 203 823 -> 793, 1024^2 colour
-// 2689 -> 2644, 720p video 5848 -> 5685.  With 16 M voxels instead 2682 and 5875 for the
-// last two; volumes beyond fill the chip at the second level too and gain nothing.
-constexpr size_t SPINS_TOGETHER = (size_t)128 << 20;
+// the spins of a volume share those launches, as many at a time as have room: each
+// spin keeps its coefficients and its lower levels' results, in at most this many bytes
+// beyond one spin's for all lanes of the context together.  The workspace has that room
+// for every volume, also those whose spins it does not hold, so it never shrinks
+// with the image: a smaller image after a larger one allocates nothing.
+//   Eight launches fewer for each pair of three-level volumes: 128 x 96 242 -> 209 us,
+// 301 x 203 823 -> 793, 1024^2 colour 2689 -> 2644, 720p video 5848 -> 5685; larger
+// volumes fill the chip at the second level too and gain nothing.
+constexpr size_t SPIN_BYTES = (size_t)256 << 20;
 
 float* run_wavelet_ht(gbm3d_ctx* c, const float* vol, int m, int n, int K, int levels, int cycleSpin,
                       const double* tau, const WaveletBank& bk, int filtType, const Spin1Cols* w = nullptr,
@@ -589,16 +592,21 @@ float* run_wavelet_ht(gbm3d_ctx* c, const float* vol, int m, int n, int K, int l
   if (m % q || n % q || K % q)
     argfail(c, "image size and numMax must be divisible by 2^levels for the 3D wavelet");
   if (cycleSpin < 1) argfail(c, "cycleSpin must be >= 1");
-  const size_t voxels = (size_t)m * n * K;
-  const bool together = !w && levels > 1 && voxels * cycleSpin <= SPINS_TOGETHER;
-  // spin s of a round of `copies`; the second level's slot pairs of all of them are one grid's z
-  const int copies = together ? std::min(cycleSpin, 65535 / (K >> 2)) : 1;
   std::vector<float*> coef(levels), rec(levels);
   std::vector<size_t> insz(levels);
+  size_t one = 0;  // floats of one spin
   for (int lv = 0; lv < levels; ++lv) {
     insz[lv] = (size_t)(m >> lv) * (n >> lv) * (K >> lv);  // 8 bands = input size
-    coef[lv] = buf<float>(c, ("ht.coef" + std::to_string(lv)).c_str(), insz[lv] * copies);
-    if (lv > 0) rec[lv] = buf<float>(c, ("ht.rec" + std::to_string(lv)).c_str(), insz[lv] * copies);
+    one += insz[lv] * (lv > 0 ? 2 : 1);
+  }
+  // spins in a round: the second level's slot pairs of all of them are one grid's z
+  const bool share = !w && levels > 1 && cycleSpin > 1;
+  const size_t room = share ? SPIN_BYTES / sizeof(float) / (c->ns.empty() ? 1 : c->lanes) : 0;
+  const int copies = share ? (int)std::min({(size_t)cycleSpin, 1 + room / one, (size_t)(65535 / (K >> 2))}) : 1;
+  for (int lv = 0; lv < levels; ++lv) {
+    const size_t extra = std::min(insz[lv] * (cycleSpin - 1), insz[lv] * room / one);
+    coef[lv] = buf<float>(c, ("ht.coef" + std::to_string(lv)).c_str(), insz[lv] + extra);
+    if (lv > 0) rec[lv] = buf<float>(c, ("ht.rec" + std::to_string(lv)).c_str(), insz[lv] + extra);
   }
   std::vector<LevelBands> th(levels);
   for (int lv = 0; lv < levels; ++lv) {

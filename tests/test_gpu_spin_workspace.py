@@ -8,6 +8,8 @@ from gbm3d_b200.api import _as_set
 
 pytestmark = pytest.mark.gpu
 
+MIB = 1 << 20
+
 
 def test_more_spins_than_a_launch_can_hold(gpu, oracle):
     """8200 spins of 8 slot pairs at the second level: more than 65535 slices of a grid."""
@@ -21,3 +23,49 @@ def test_more_spins_than_a_launch_can_hold(gpu, oracle):
     U, W = gpu.denoiseAndAggregateGPU(V, _as_set(S), tau, Psi, Psi2, o)
     Uo, Wo = oracle.denoiseAndAggregateGPU(V, S, tau, o, filters=oracle.haar_filters(), prec=32)
     assert np.array_equal(U, Uo) and np.array_equal(W, Wo)
+
+
+def _dense(cycles):
+    o = options.resolve_opts({"profile": "default"})
+    o.update(blockSize=8, blockSizeWie=8, matchSize=32, refStride=3, refStrideWie=3, matchSpins=[0], matchSpinsWie=[0],
+             cycleSpin=cycles, Wiener=False)
+    return o
+
+
+def _step1(ctx, m, n, cycles, seed=1):
+    """Step 1 of a random device image; the device memory in use after it."""
+    import torch
+    from gbm3d_b200 import api
+    x = 255 * torch.rand((n, m), dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(seed))
+    out = torch.empty_like(x)
+    torch.cuda.synchronize()
+    api.GBM3D_device(x.data_ptr(), m, n, 25.0, out.data_ptr(), _dense(cycles), ctx=ctx)
+    ctx.synchronize()
+    res = out.cpu()
+    del x, out
+    torch.cuda.empty_cache()
+    free, total = torch.cuda.mem_get_info()
+    return total - free, res
+
+
+def test_workspace_of_a_smaller_image_is_that_of_the_larger(gpu):
+    """A smaller image after a larger one allocates nothing (a growth would stall every stream
+    and drop the captured graph)."""
+    from gbm3d_b200._lib import Context
+    ctx = Context(0)
+    used, _ = _step1(ctx, 800, 800, 2)
+    for side in (700, 500, 250):
+        assert _step1(ctx, side, side, 2)[0] == used
+    ctx.close()
+
+
+@pytest.mark.parametrize("cycles,side", [(2, 750), (8, 370)])
+def test_shared_spins_memory_is_bounded(gpu, cycles, side):
+    from gbm3d_b200._lib import Context
+    used = {}
+    for c in (1, cycles):
+        ctx = Context(0)
+        base = _step1(ctx, 40, 40, 1)[0]
+        used[c] = _step1(ctx, side, side, c)[0] - base
+        ctx.close()
+    assert used[cycles] - used[1] <= 256 * MIB + 16 * MIB  # 16: pages of the few buffers
