@@ -68,6 +68,8 @@ struct gbm3d_ctx {
   std::vector<cudaStream_t> lane_st;
   std::vector<cudaEvent_t> lane_ev;  // [0] fork, [1 + l] lane l done
   std::string ns;
+  bool spin_no_room = false;  // an allocation failed: cycle spins one at a time from now on (run_wavelet_ht)
+  size_t allocs = 0;          // workspace allocations so far
 };
 
 namespace {
@@ -82,6 +84,7 @@ void set_err(gbm3d_ctx* c, const std::string& s) {
 
 void ck(gbm3d_ctx* c, cudaError_t e, const char* what) {
   if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here, not by the next call's first launch
     set_err(c, std::string(what) + ": " + cudaGetErrorString(e));
     throw Fail{e == cudaErrorMemoryAllocation ? GBM3D_ERR_NOMEM : GBM3D_ERR_CUDA};
   }
@@ -101,6 +104,27 @@ void report_flag(gbm3d_ctx* c, int flag) {
   if (flag & 4) argfail(c, "matcher: a search-window TMA copy did not complete within its wait limit", GBM3D_ERR_CUDA);
 }
 
+bool spin_buffer(const std::string& name) {
+  return name.find("ht.coef") != std::string::npos || name.find("ht.rec") != std::string::npos;
+}
+
+// Gives back the wavelet buffers, which hold room for several cycle spins, the first time an
+// allocation fails; run_wavelet_ht then takes them anew for one spin.
+bool release_spins(gbm3d_ctx* c) {
+  if (c->spin_no_room) return false;
+  c->spin_no_room = true;
+  c->graph_key.clear();
+  for (auto it = c->bufs.begin(); it != c->bufs.end();) {
+    if (!spin_buffer(it->first)) {
+      ++it;
+      continue;
+    }
+    cudaFree(it->second.first);
+    it = c->bufs.erase(it);
+  }
+  return true;
+}
+
 template <class T>
 T* buf(gbm3d_ctx* c, const char* cname, size_t count) {
   const size_t bytes = std::max<size_t>(count * sizeof(T), 256);
@@ -112,8 +136,14 @@ T* buf(gbm3d_ctx* c, const char* cname, size_t count) {
     cudaFree(it->second.first);
     c->bufs.erase(it);
   }
+  ++c->allocs;
   void* p = nullptr;
-  ck(c, cudaMalloc(&p, bytes), name.c_str());
+  cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation && release_spins(c) && !spin_buffer(name)) {
+    cudaGetLastError();
+    e = cudaMalloc(&p, bytes);
+  }
+  ck(c, e, name.c_str());
   c->bufs[name] = {p, bytes};
   return reinterpret_cast<T*>(p);
 }
@@ -599,15 +629,24 @@ float* run_wavelet_ht(gbm3d_ctx* c, const float* vol, int m, int n, int K, int l
     insz[lv] = (size_t)(m >> lv) * (n >> lv) * (K >> lv);  // 8 bands = input size
     one += insz[lv] * (lv > 0 ? 2 : 1);
   }
-  // spins in a round: the second level's slot pairs of all of them are one grid's z
-  const bool share = !w && levels > 1 && cycleSpin > 1;
-  const size_t room = share ? SPIN_BYTES / sizeof(float) / (c->ns.empty() ? 1 : c->lanes) : 0;
-  const int copies = share ? (int)std::min({(size_t)cycleSpin, 1 + room / one, (size_t)(65535 / (K >> 2))}) : 1;
-  for (int lv = 0; lv < levels; ++lv) {
-    const size_t extra = std::min(insz[lv] * (cycleSpin - 1), insz[lv] * room / one);
-    coef[lv] = buf<float>(c, ("ht.coef" + std::to_string(lv)).c_str(), insz[lv] + extra);
-    if (lv > 0) rec[lv] = buf<float>(c, ("ht.rec" + std::to_string(lv)).c_str(), insz[lv] + extra);
+  auto workspace = [&](size_t room) {  // room: floats beyond one spin's
+    for (int lv = 0; lv < levels; ++lv) {
+      const size_t extra = std::min(insz[lv] * (cycleSpin - 1), insz[lv] * room / one);
+      coef[lv] = buf<float>(c, ("ht.coef" + std::to_string(lv)).c_str(), insz[lv] + extra);
+      if (lv > 0) rec[lv] = buf<float>(c, ("ht.rec" + std::to_string(lv)).c_str(), insz[lv] + extra);
+    }
+  };
+  size_t room = !w && levels > 1 && !c->spin_no_room ? SPIN_BYTES / sizeof(float) / (c->ns.empty() ? 1 : c->lanes) : 0;
+  try {
+    workspace(room);
+  } catch (const Fail& f) {
+    if (f.code != GBM3D_ERR_NOMEM || room == 0) throw;
+    c->err.clear();
+    workspace(room = 0);  // buf() has given back what there was
   }
+  // spins in a round: the second level's slot pairs of all of them are one grid's z
+  const int copies =
+      room ? (int)std::min({(size_t)cycleSpin, 1 + room / one, (size_t)(65535 / (K >> 2))}) : 1;
   std::vector<LevelBands> th(levels);
   for (int lv = 0; lv < levels; ++lv) {
     th[lv].tau[0] = 0.f;
@@ -2087,6 +2126,7 @@ void run_graph(gbm3d_ctx* c, const std::string& key, bool use_graph, F&& run_all
   }
   run_all();
   const bool tm = c->timing;
+  const size_t allocs = c->allocs;
   c->timing = false;
   ck(c, cudaStreamBeginCapture(c->st, cudaStreamCaptureModeRelaxed), "cudaStreamBeginCapture");
   cudaGraph_t g = nullptr;
@@ -2103,6 +2143,10 @@ void run_graph(gbm3d_ctx* c, const std::string& key, bool use_graph, F&& run_all
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   c->graph_exec = nullptr;
   c->graph_key.clear();
+  if (c->allocs != allocs) {  // a buffer moved under the capture (release_spins): the next call captures
+    cudaGraphDestroy(g);
+    return;
+  }
   const cudaError_t e = cudaGraphInstantiate(&c->graph_exec, g, 0);
   cudaGraphDestroy(g);
   ck(c, e, "cudaGraphInstantiate");

@@ -69,3 +69,42 @@ def test_shared_spins_memory_is_bounded(gpu, cycles, side):
         used[c] = _step1(ctx, side, side, c)[0] - base
         ctx.close()
     assert used[cycles] - used[1] <= 256 * MIB + 16 * MIB  # 16: pages of the few buffers
+
+
+@pytest.mark.parametrize("wiener,graph", [(False, False), (True, False), (True, True)])
+def test_device_without_room_for_the_shared_spins(gpu, wiener, graph):
+    """With too little memory left for them (at their own allocation, or with the second step's at a
+    later one) the spins run one after another, to the same result, and the context goes on working."""
+    import torch
+    from gbm3d_b200 import api
+    from gbm3d_b200._lib import Context
+    side = 600
+    o = dict(_dense(3), Wiener=wiener)
+    x = 255 * torch.rand((side, side), dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    out = torch.empty_like(x)
+
+    def run(ctx):
+        out.zero_()
+        api.GBM3D_batch([x], [25.0], o, ctx=ctx, use_graph=graph, outputs=[out])
+        return ctx.launch_count(), out.cpu()
+
+    def free():
+        torch.cuda.empty_cache()
+        return torch.cuda.mem_get_info()[0]
+
+    start = free()
+    ctx = Context(0)
+    _, want = run(ctx)
+    need = start - free()
+    ctx.close()
+    ctx = Context(0)
+    hold = torch.empty(free() - (need - 128 * MIB), dtype=torch.uint8, device="cuda")
+    try:
+        got = [run(ctx) for _ in range(3)]
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    for launches, u in got + [run(ctx)]:
+        assert torch.equal(u, want)
+    assert not graph or got[2][0] == 1  # the second call at the latest was captured
+    ctx.close()
