@@ -31,8 +31,8 @@ __host__ __device__ __forceinline__ int pad_index(int r, int L, int h) {
 // First statement of every kernel that launch_next() launches: wait until the
 // kernels before it on the stream are complete and their writes visible, then
 // let the next one's CTAs take the slots that this one leaves free.  The pointers
-// given are those read through __ldg or as const __restrict__ parameters: loads that
-// the compiler may take for constant over the kernel and move up.  They leave here with
+// given are those read through __ldg and the __restrict__ parameters that are read: loads
+// that the compiler may take for untouched by the wait and move up.  They leave here with
 // a value of unknown origin, so that no such load can be made before the wait.
 template <class... P>
 __device__ __forceinline__ void begin_after_previous(P&... read_only) {

@@ -379,7 +379,7 @@ __global__ void k_or_flag(const int* __restrict__ flag, int* __restrict__ sticky
 
 __global__ void k_accum2(const float* __restrict__ u, const float* __restrict__ w, int Mp, int Np, int s,
                          double* __restrict__ ua, double* __restrict__ wa, int first) {
-  begin_after_previous(u, w);
+  begin_after_previous(u, w, ua, wa);
   const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
   if (r >= Mp || c >= Np) return;
   const size_t src = shift_index(r, s, Mp) + (size_t)shift_index(c, s, Np) * Mp;
