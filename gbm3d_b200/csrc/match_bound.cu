@@ -311,7 +311,22 @@ __global__ void __launch_bounds__(128, 6) k_match_bound(const __grid_constant__ 
     }
   }
   int count = K;
-  if (!listed) count = search_exhaustive<D, D2>(A, wv, scr, lane);
+  if (!listed) {
+    // an overflow may be a window of one value (an empty border, a mask, saturation): every
+    // distance is exactly zero and the lowest indices win
+    bool differs = big;
+    const uint32_t w0 = __float_as_uint(wv[0]);
+    for (int c = 0; c < WD && !__any_sync(FULL, differs); ++c) {
+      const float* col = wv + c * WP;
+      differs = __float_as_uint(col[lane]) != w0 || (lane < WD - 32 && __float_as_uint(col[32 + lane]) != w0);
+    }
+    if (__any_sync(FULL, differs)) {
+      count = search_exhaustive<D, D2>(A, wv, scr, lane);
+    } else {
+      if (lane < K) scr[64 + lane] = lane == 0 ? (uint32_t)(H + H * D2 + 1) : (uint32_t)lane + 1;
+      __syncwarp();
+    }
+  }
   emit_group<D, D2>(A, g, i, j, wv, scr + 64, count, lane);
 }
 

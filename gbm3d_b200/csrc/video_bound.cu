@@ -224,8 +224,28 @@ __global__ void __launch_bounds__(128, OCC) k_match_video_bound(VideoMatchArgs A
   __syncthreads();
   const int C = cnt;
   const bool redo = big || C < K || C > LCAND;
-  if (tid == 0) A.redo[g] = redo ? 1 : 0;
-  if (redo) return;
+  const size_t mn = (size_t)A.m * A.n;
+  if (redo) {
+    // an overflow may be windows of one value (black bars, a mask): every distance is exactly
+    // zero and the lowest indices win
+    const float w0 = A.pads[0][(size_t)(i * D) + (size_t)(j * D) * A.P];
+    bool same = !big;  // the same for every thread
+    for (int f = 0; f < F && same; ++f) {
+      stage(f);
+      bool differs = false;
+      for (int e = tid; e < WD * WD; e += 128)
+        differs |= __float_as_uint(win[(e >> 6) * WP + (e & 63)]) != __float_as_uint(w0);
+      same = !__syncthreads_or(differs);
+    }
+    if (tid == 0) A.redo[g] = same ? 0 : 1;
+    if (same) {
+      if (tid < K) A.S[(size_t)g * K + tid] = (uint32_t)(tid == 0 ? DD * F / 2 + H : tid) + 1;
+      for (int e = tid; e < K * DD; e += 128)
+        A.volume[(size_t)(i * D + e % D) + (size_t)A.m * (j * D + (e / D) % D) + mn * (e / DD)] = w0;
+    }
+    return;
+  }
+  if (tid == 0) A.redo[g] = 0;
 
   // ---- exact SSD of the candidates, frame by frame, in the direct kernel's
   // operation order (row-major, t = x - w, acc = fmaf(t, t, acc))
@@ -268,7 +288,6 @@ __global__ void __launch_bounds__(128, OCC) k_match_video_bound(VideoMatchArgs A
   __syncthreads();
   if (tid < K) A.S[(size_t)g * K + tid] = sel[tid] + 1;
   // Volume(i d + r, j d + c, k): the selected block, image-shaped m x n x K
-  const size_t mn = (size_t)A.m * A.n;
   for (int e = tid; e < K * DD; e += 128) {
     const int k = e / DD, r = e % D, c = (e / D) % D;
     const uint32_t s = sel[k];
