@@ -289,6 +289,7 @@ static cudaError_t launch_px_cap(const AggArgs& A, cudaStream_t st) {
 //   Bounds at 1024^2 dense (ncu): shared-memory pipe 61 %, issue 42-50 %, DRAM
 // 33 %; 272 us per launch against 625 us pixel at a time (of which the
 // group-major layout with its prefetch 310: DRAM reads 2.07 -> 0.72 GB).
+
 // N floats at p (a multiple of 128 bytes) on their way to L2: an entry's block
 // is loaded only when the list is walked.
 template <int N>
@@ -308,7 +309,8 @@ struct AggBlk {
   static constexpr int NT = TWO ? 64 : 32;
   static constexpr int LC = (TWO ? 96 : 128) + 32 * EB;  // list capacity
   static constexpr int LISTS = (TWO ? 2 : 1) * (LC + 2 * NB);
-  static constexpr size_t BYTES = (size_t)LISTS * sizeof(int4) + (size_t)PT * COLS * SV * sizeof(float);
+  static constexpr int CELLS4 = (PT * COLS * SV + 3) / 4;  // the sums in 16-byte words
+  static constexpr size_t BYTES = (size_t)LISTS * sizeof(int4) + (size_t)CELLS4 * sizeof(float4);
   static_assert(PT >= RR + 2 * D - 1, "pitch");
 };
 
@@ -329,7 +331,7 @@ __global__ void __launch_bounds__(AggBlk<D, KAHAN, RR, RC>::NT) k_aggregate_blk(
   int4* lst = smv;
   float* acc = reinterpret_cast<float*>(smv + G::LISTS);
   const unsigned FULL = 0xffffffffu, below = (1u << lane) - 1u;
-  for (int e = threadIdx.x; e < PT * G::COLS * SV / 4; e += G::NT) reinterpret_cast<float4*>(acc)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int e = threadIdx.x; e < G::CELLS4; e += G::NT) reinterpret_cast<float4*>(acc)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
 
   const int tiles_r = (A.m + RR - 1) / RR, tiles_c = (A.n + RC - 1) / RC;
   const int tcol = (int)(blockIdx.x / tiles_r) + A.ct0;  // the window's column tiles, modulo the count

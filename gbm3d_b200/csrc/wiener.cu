@@ -299,6 +299,7 @@ __global__ void __launch_bounds__(128) k_wiener(WienerArgs A) {
 // instructions per group); 1024^2 dense 1.06 -> 0.80 ms (two spins).  Now at 87 % of the
 // shared-memory pipe; 326 of 840 wavefronts per group are the gather, four
 // lines per 4-byte asynchronous copy (through registers: the same).
+
 // out[q] = sum_j M(q, j) v[j] (M column-major 8 x 8, a constant operand), each a serial
 // fmaf chain from 0 in ascending j, two rows per packed instruction
 __device__ __forceinline__ void mat8(const float* M, const float (&v)[8], float (&out)[8]) {
