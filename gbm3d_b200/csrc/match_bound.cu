@@ -33,8 +33,8 @@
 // candidates, 85 + 40 for the rounded window and the norm sums).
 //   Where the list overflows the bound is paid on top of the exhaustive search, so
 // windows of one value, whose distances are all zero, are told from the rest there
-// (2048^2 at strides 8 / 6, both steps: a flat image 1.79 -> 1.24 ms, the exhaustive matcher
-// 1.29; one half masked 1.32 -> 0.60 against 1.33; noisy 0.55 against 1.05).
+// (2048^2 at strides 8 / 6, both steps: a flat image 1.79 -> 1.26 ms, the exhaustive matcher
+// 1.29; one half masked 1.32 -> 0.63 against 1.33; noisy 0.55 against 1.05).
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -58,6 +58,17 @@ constexpr int LCAND = 128;                                  // candidates a warp
 // 32-bit words of a warp's scratch: the exhaustive search's 224, or 64 (reference
 // block, row-major) + 32 (S) + 2 LCAND (keys and indices)
 constexpr int SCR = 96 + 2 * LCAND;
+
+// Whether a reference's window holds one value throughout.  A call, and only where the whole window is
+// within the bound: inlined it costs every reference 1 % by the code around it.
+__device__ __noinline__ bool one_value(const float* wv, int lane) {
+  uint32_t differs = 0;
+#pragma unroll 1
+  for (int c = 0; c < WD; ++c)
+    differs |= (__float_as_uint(wv[c * WP + lane]) ^ __float_as_uint(wv[0])) |
+               (__float_as_uint(wv[c * WP + WD - 32 + lane]) ^ __float_as_uint(wv[0]));
+  return !__any_sync(0xffffffffu, differs);
+}
 
 // Groups of the column range [j0, j0 + nj): blockIdx.x = i + M (tile of four columns).
 __global__ void __launch_bounds__(128, 6) k_match_bound(const __grid_constant__ CUtensorMap tmap, MatchArgs A, int j0,
@@ -253,6 +264,14 @@ __global__ void __launch_bounds__(128, 6) k_match_bound(const __grid_constant__ 
       for (int e = 0; e < 32; ++e) hits |= acc[e >> 4][(e >> 2) & 3][e & 3] >= th ? 1u << e : 0u;
       C = __reduce_add_sync(FULL, __popc(hits));
     }
+    if (C == D2 * D2 && one_value(wv, lane)) {
+      // every distance is exactly zero and the lowest indices win: column 0's first K rows
+      hits = 0;
+#pragma unroll
+      for (int e = 0; e < 16; ++e)
+        if (!(e & 2) && gq == 0 && 8 * (e >> 2) + 4 * (e & 1) + t < K) hits |= 1u << e;
+      C = K;
+    }
     if (C >= K && C <= LCAND) {
       listed = true;
       float* xrow = reinterpret_cast<float*>(scr);
@@ -314,22 +333,7 @@ __global__ void __launch_bounds__(128, 6) k_match_bound(const __grid_constant__ 
     }
   }
   int count = K;
-  if (!listed) {
-    // an overflow may be a window of one value (an empty border, a mask, saturation): every
-    // distance is exactly zero and the lowest indices win
-    bool differs = big;
-    const uint32_t w0 = __float_as_uint(wv[0]);
-    for (int c = 0; c < WD && !__any_sync(FULL, differs); ++c) {
-      const float* col = wv + c * WP;
-      differs = __float_as_uint(col[lane]) != w0 || (lane < WD - 32 && __float_as_uint(col[32 + lane]) != w0);
-    }
-    if (__any_sync(FULL, differs)) {
-      count = search_exhaustive<D, D2>(A, wv, scr, lane);
-    } else {
-      if (lane < K) scr[64 + lane] = lane == 0 ? (uint32_t)(H + H * D2 + 1) : (uint32_t)lane + 1;
-      __syncwarp();
-    }
-  }
+  if (!listed) count = search_exhaustive<D, D2>(A, wv, scr, lane);
   emit_group<D, D2>(A, g, i, j, wv, scr + 64, count, lane);
 }
 
