@@ -204,19 +204,23 @@ def padded_side(o) -> int:
 # where the step-1 grid has 340 x 340 references and the step-2 grid the same.  A launch's traffic grows with its
 # reference count, so it is scaled by the workload's count.  Wavelet kernels:
 # the level-0 launch (the one the bytes describe).
-TRAFFIC_1024 = {"match": 432.4e6, "wav_synthesis": 909.4e6, "wav_analysis": 909.1e6, "aggregate": 1065.1e6,
-                "wiener": 463.9e6, "ht_weights": 478.2e6}
+TRAFFIC_1024 = {"match": 428.6e6, "wav_synthesis": 946.0e6, "wav_analysis": 928.1e6, "aggregate": 731.4e6,
+                "wiener": 455.8e6, "ht_weights": 474.5e6}
 REFS_1024 = 340 * 340
 # The same (bytes per launch, averaged over the family's launches of one call)
 # for the option sets the autotuner picks, each captured on a 2048 x 2048 image
 # (padded side given); a launch's traffic grows with the padded image area.
 # Key: refStride, refStrideWie, matchSpins, matchSpinsWie, cycleSpin, matchSize.
 TRAFFIC_TUNED_2048 = {
-    (8, 6, (0,), (0,), 1, 32): (2048, {"match": 125.1e6, "wav_analysis": 177.0e6, "wav_synthesis": 177.6e6,
-                                       "ht_weights": 269.2e6, "aggregate": 419.8e6, "wiener": 488.1e6}),
-    (8, 7, (0,), (0,), 1, 32): (2080, {"match": 131.6e6, "wav_analysis": 183.3e6, "wav_synthesis": 183.8e6,
-                                       "ht_weights": 277.5e6, "aggregate": 363.9e6, "wiener": 365.3e6}),
+    (8, 6, (0,), (0,), 1, 32): (2048, {"match": 125.2e6, "wav_analysis": 180.2e6, "wav_synthesis": 190.2e6,
+                                       "ht_weights": 269.6e6, "aggregate": 486.6e6, "wiener": 484.7e6}),
+    (8, 7, (0,), (0,), 1, 32): (2080, {"match": 129.9e6, "wav_analysis": 186.5e6, "wav_synthesis": 196.0e6,
+                                       "ht_weights": 277.6e6, "aggregate": 380.5e6, "wiener": 361.6e6}),
 }
+# Shared-memory wavefronts per reference of the bounded matcher (patch 8, search 32), from the
+# same captures (l1tex__data_pipe_lsu_wavefronts_mem_shared.sum over the references): step 1
+# with the volume's gather, step 2.  By step-1 stride.
+MATCH_WAVEFRONTS = {3: (696, 569), 8: (717, 609)}
 
 
 def roofline(o, ktimes, peaks, sm_mhz):
@@ -254,10 +258,19 @@ def roofline(o, ktimes, peaks, sm_mhz):
                                                         "two padded images once"),
         "ht_weights": ("hbm", nS * (4 * V + 4 * G1), "read the denoised volume once"),
         "match": ("fp32", nS * G1 * d2 * d2 * d * d * 3 + nW * G2 * d2 * d2 * dw * dw * 3,
-                  "N_ref * W^2 * d^2 * 3 (sub, mul, add of the exact SSD)"),
+                  "N_ref * W^2 * d^2 * 3 (sub, mul, add of the exact SSD of every candidate, which a search bounded "
+                  "by tensor-core distances leaves out for most: nominal there)"),
         "match_tc": ("tensor", (nS * G1 + nW * G2) * d2 * d2 * 64 * 2,
                      "2 N_ref W^2 d^2 (the a.b products each reference needs; d = 8)"),
     }
+    # the bounded matcher: f16 products on the tensor cores and a few exact distances, limited by
+    # the shared-memory pipe (one wavefront per SM and cycle); its time is the match family's
+    bounded = d == dw == 8 and d2 == 32 and o["numMin"] == K
+    if bounded and "match" in ktimes:
+        w1, w2 = MATCH_WAVEFRONTS.get(s1, MATCH_WAVEFRONTS[8])
+        work["match_bound"] = ("smem", nS * G1 * w1 + nW * G2 * w2,
+                               f"N_ref * {w1} (step 1) and {w2} (step 2) shared-memory wavefronts, counted by ncu")
+        ktimes = dict(ktimes, match_bound=ktimes["match"])
     out = {}
     for f, (bound, amount, what) in work.items():
         if f not in ktimes:
@@ -267,14 +280,16 @@ def roofline(o, ktimes, peaks, sm_mhz):
             ach, peak, unit = amount / (ms / 1e3) / 1e9, hbm, "GB/s"
         elif bound == "tensor":
             ach, peak, unit = amount / (ms / 1e3) / 1e12, peaks.get("bf16_tflops") or 1590.0, "TFLOP/s"
+        elif bound == "smem":
+            ach, peak, unit = amount / (ms / 1e3) / 1e9, 148 * sm_mhz * 1e6 / 1e9, "Gwavefront/s"
         else:
             ach, peak, unit = amount / (ms / 1e3) / 1e12, fp32, "TFLOP/s"
         out[f] = {"bound": bound, "achieved": ach, "peak": peak, "unit": unit, "frac": ach / peak,
                   "ms_per_step": ms, "launches": n, "algorithmic_per_step": amount, "what": what}
     if not out:
         return None, out
-    top = max(out, key=lambda f: out[f]["ms_per_step"])
-    r = out[top]
+    top = max((f for f in out if f != "match_bound"), key=lambda f: out[f]["ms_per_step"])
+    r = out["match_bound"] if top == "match" and bounded else out[top]
     key = (s1, s2, tuple(o["matchSpins"]), tuple(o["matchSpinsWie"]), cs, d2)
     if key in TRAFFIC_TUNED_2048:
         side, table = TRAFFIC_TUNED_2048[key]
@@ -291,6 +306,7 @@ def roofline(o, ktimes, peaks, sm_mhz):
             "frac": r["frac"], "traffic": traffic, "traffic_source": tsrc,
             "peak_source": {"hbm": "MEASURED_PEAKS.json hbm_gbs (of measured)",
                             "tensor": "MEASURED_PEAKS.json bf16_tflops (of measured)",
+                            "smem": "derived: 148 SMs x 1 wavefront per cycle x median SM clock under load",
                             "fp32": "derived: 148 SMs x 128 FP32 lanes x 2 flop x median SM clock under load"}[r["bound"]],
             "algorithmic_per_step": r["algorithmic_per_step"], "launches_per_step": r["launches"],
             "what": r["what"]}
