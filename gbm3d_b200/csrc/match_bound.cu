@@ -28,9 +28,10 @@
 // Measured against the exhaustive matcher (B200, both steps of one call):
 // 4096^2 at strides 8 / 7 3.29 -> 1.80 ms, dense (stride 3, two spins) 40.1 ->
 // 21.3 ms, 1677 x 1531 at stride 3 4.73 -> 2.4 ms.  About 1.8 k warp instructions
-// per reference instead of 5.7 k; bound by the shared-memory pipe, not by issue
-// (wavefronts per reference: 160 ldmatrix, about 165 exact-SSD loads of scattered
-// candidates, 85 + 40 for the rounded window and the norm sums).
+// per reference instead of 5.7 k; bound by the shared-memory pipe (82-92 % of the
+// cycles: 570-720 wavefronts per reference, of them 160 ldmatrix, about 165 exact-SSD
+// loads of scattered candidates, 85 + 40 for the rounded window and the norm sums), not by
+// issue (56-60 %).
 //   Where the list overflows the bound is paid on top of the exhaustive search, so
 // windows of one value, whose distances are all zero, are told from the rest there
 // (2048^2 at strides 8 / 6, both steps: a flat image 1.79 -> 1.26 ms, the exhaustive matcher

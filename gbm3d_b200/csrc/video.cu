@@ -136,8 +136,7 @@ __global__ void __launch_bounds__(128) k_match_video(VideoMatchArgs A) {
 // thread steps through the list for its four pixels of one row; each term fl(w block)
 // is added in double (the reference's U and out.K are double arrays).  A thread
 // per pixel testing every (reference, slot) pair of its neighbourhood took 233 us
-// for three 720p frames; this 74
-// (entries' loads four at a time ahead of the adds: 84).  A list that could overflow is applied and
+// for three 720p frames; this 67 (entries' loads four at a time ahead of the adds: 77).  A list that could overflow is applied and
 // refilled, so any capacity gives the same sums.
 //   With Y, the sums are added to the call's single-precision accumulators, as
 // VBM3D.m:52-56 does after each window, instead of being written out.

@@ -12,8 +12,10 @@
 //   One CTA of four warps per reference; frames pass one after another through
 // one window buffer (33 KB: six CTAs per SM), the distances stay in registers,
 // and the frames that hold candidates are staged once more for the exact SSD.
-//   720p, F = 3: 307 -> 130 us per window; 17.7 k shared-memory wavefronts per
-// reference (4.6 k ldmatrix, 7 k the exact SSDs), barriers while one warp ranks.
+//   720p, F = 3: 307 -> 130 us per window; 17.5 k shared-memory wavefronts per
+// reference (4.6 k ldmatrix, 7 k the exact SSDs), barriers while one warp ranks.  The
+// 32 row and column sums of a thread cross barriers in registers, and some spill (F = 3: 56
+// bytes of stores at the 80 registers that six CTAs allow).
 // References whose list overflows, or whose values leave the f16 range, are
 // marked in A.redo for the direct kernel.
 #include "bound.cuh"
