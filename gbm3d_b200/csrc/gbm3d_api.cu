@@ -114,6 +114,7 @@ bool release_spins(gbm3d_ctx* c) {
   if (c->spin_no_room) return false;
   c->spin_no_room = true;
   c->graph_key.clear();
+  cudaDeviceSynchronize();  // the other lanes' kernels may still use theirs
   for (auto it = c->bufs.begin(); it != c->bufs.end();) {
     if (!spin_buffer(it->first)) {
       ++it;
